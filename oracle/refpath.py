@@ -16,8 +16,7 @@ _DEFAULT_MOUNT = "/root/reference"
 
 
 def reference_root():
-    """The reference checkout's root directory, or None when it is absent."""
-    r = os.environ.get("SUNDOG_REFERENCE")
-    if r:
-        return r if os.path.isdir(r) else None
-    return _DEFAULT_MOUNT if os.path.isdir(_DEFAULT_MOUNT) else None
+    """The reference checkout's root directory, or None when it is absent (an
+    empty mount point counts as absent: there is nothing in it to compile)."""
+    r = os.environ.get("SUNDOG_REFERENCE") or _DEFAULT_MOUNT
+    return r if os.path.isfile(os.path.join(r, "src", "capi_scene.cpp")) else None
