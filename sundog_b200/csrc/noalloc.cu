@@ -70,8 +70,8 @@ __global__ void ptTileSetup(SdLaunch lp, TileSpec t) {
 __device__ __forceinline__ unsigned long long fullFrameId(const SdLaunch& lp, int px, int py,
                                                           int sLocal) {
   int tile = (py >> 3) * lp.tilesX + (px >> 3);
-  int rem = tile * 64 + (py & 7) * 8 + (px & 7);
-  return (unsigned long long)sLocal * lp.npixPad + rem;
+  int rem = tile * 64 + tileIndex(px & 7, py & 7);
+  return (unsigned long long)rem * lp.sppThisLaunch + sLocal;
 }
 
 __global__ void __launch_bounds__(kRenderBlock) ptTileNoAlloc() {
@@ -84,8 +84,9 @@ __global__ void __launch_bounds__(kRenderBlock) ptTileNoAlloc() {
   const long long total = (long long)npt * t.sampleCount;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
-    int sLocal = (int)(i / npt);
-    int rem = (int)(i - (long long)sLocal * npt);
+    // The samples of a pixel are consecutive (total is at most kTileSlots).
+    int rem = (int)i / t.sampleCount;
+    int sLocal = (int)i - rem * t.sampleCount;
     int px = t.x0 + rem % t.w, py = t.y0 + rem / t.w;
     Path p;
     if (!startPath(lp, fullFrameId(lp, px, py, sLocal), p)) continue;
@@ -108,7 +109,7 @@ __global__ void ptTileFold() {
   if (i >= npt) return;
   float4 acc = t.film[i];
   for (int k = 0; k < t.sampleCount; k++) {
-    float4 x = lp.sampleL[(size_t)k * npt + i];
+    float4 x = lp.sampleL[(size_t)i * t.sampleCount + k];
     int s1 = t.sampleBegin + k + 1;
     acc = make_float4(acc.x + (x.x - acc.x) / s1, acc.y + (x.y - acc.y) / s1,
                       acc.z + (x.z - acc.z) / s1, 1.0f);

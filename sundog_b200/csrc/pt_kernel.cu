@@ -4,8 +4,8 @@
 // a lane whose path ends writes that sample's radiance to the per-sample
 // buffer and immediately takes the next path index (one warp-aggregated
 // atomicAdd per refill), so lanes stay busy while long paths finish. A path
-// index maps to (sample, pixel) with the sample outermost and pixels in 8x8
-// tiles, so a warp starts on an 8x4 block of neighbouring camera rays.
+// index maps to (pixel, sample) with the sample innermost and pixels in 8x8
+// tiles, so a warp starts on the camera rays of one pixel or a small patch.
 //
 // ptFold: folds the per-sample values into the film in sample order with the
 // reference's running mean acc += (x - acc) / (s + 1) (device/programs.cu:
@@ -102,7 +102,7 @@ __global__ void ptFold() {
   }
   float4 acc = lp.accum[pix];
   for (int i = 0; i < lp.sppThisLaunch; i++) {
-    float4 x = lp.sampleL[(size_t)i * npix + pix];
+    float4 x = lp.sampleL[(size_t)pix * lp.sppThisLaunch + i];
     int s1 = lp.sampleOffset + i + 1;
     acc = make_float4(acc.x + (x.x - acc.x) / s1, acc.y + (x.y - acc.y) / s1,
                       acc.z + (x.z - acc.z) / s1, 1.0f);
@@ -111,7 +111,7 @@ __global__ void ptFold() {
   if (!lp.aovOn) return;
   float4 al = lp.aovAlbedo[pix], nm = lp.aovNormal[pix];
   for (int i = 0; i < lp.sppThisLaunch; i++) {
-    size_t k = (size_t)i * npix + pix;
+    size_t k = (size_t)pix * lp.sppThisLaunch + i;
     float4 a = lp.sampleAlb[k], n = lp.sampleNrm[k];
     int s1 = lp.sampleOffset + i + 1;
     al = make_float4(al.x + (a.x - al.x) / s1, al.y + (a.y - al.y) / s1, al.z + (a.z - al.z) / s1, 1.0f);

@@ -98,34 +98,49 @@ __device__ __forceinline__ void startPathAt(const SdLaunch& lp, int px, int py, 
   p.depth = 0;
 }
 
+// Pixel `w` of an 8x8 tile in Morton order, so any aligned run of a power of
+// two of them is a compact patch, and back.
+__device__ __forceinline__ int tileX(int w) { return (w & 1) | ((w >> 1) & 2) | ((w >> 2) & 4); }
+__device__ __forceinline__ int tileY(int w) { return tileX(w >> 1); }
+__device__ __forceinline__ int tileIndex(int x, int y) {
+  return (x & 1) | ((y & 1) << 1) | ((x & 2) << 1) | ((y & 2) << 2) | ((x & 4) << 2) |
+         ((y & 4) << 3);
+}
+
+// Splits a path index into (tile-ordered pixel, sample of `spp`): the samples
+// of a pixel are consecutive, so a warp holds the samples of one pixel (or of
+// a small patch when spp < 32) and its camera rays visit the same nodes,
+// textures and materials.
+__device__ __forceinline__ void splitPathId(unsigned long long id, int spp, int& pixel, int& s) {
+  if (id < (1ull << 32)) {  // a 32-bit division: the common case, far cheaper
+    const unsigned id32 = (unsigned)id;
+    pixel = (int)(id32 / (unsigned)spp);
+    s = (int)(id32 - (unsigned)pixel * (unsigned)spp);
+  } else {
+    pixel = (int)(id / (unsigned long long)spp);
+    s = (int)(id - (unsigned long long)pixel * spp);
+  }
+}
+
 // Camera sample for path index id; false if the index is tile padding.
 __device__ __forceinline__ bool startPath(const SdLaunch& lp, unsigned long long id, Path& p) {
-  int sLocal, px, py;
+  int rem, sLocal, px, py;
+  splitPathId(id, lp.sppThisLaunch, rem, sLocal);
+  const int within = rem & 63;
   if (lp.shardCount > 1) {
-    sLocal = (int)(id / (unsigned long long)lp.shardPad);
-    int rem = (int)(id - (unsigned long long)sLocal * lp.shardPad);
     int tile = (rem >> 12) * lp.shardCount + lp.shardIndex;
-    int block = (rem >> 6) & 63, within = rem & 63;
-    px = (tile % lp.shardTilesX) * 64 + (block & 7) * 8 + (within & 7);
-    py = (tile / lp.shardTilesX) * 64 + (block >> 3) * 8 + (within >> 3);
+    int block = (rem >> 6) & 63;
+    px = (tile % lp.shardTilesX) * 64 + (block & 7) * 8 + tileX(within);
+    py = (tile / lp.shardTilesX) * 64 + (block >> 3) * 8 + tileY(within);
   } else {
-    int rem;
-    if (id < (1ull << 32)) {  // a 32-bit division: the common case, far cheaper
-      const unsigned id32 = (unsigned)id;
-      sLocal = (int)(id32 / (unsigned)lp.npixPad);
-      rem = (int)(id32 - (unsigned)sLocal * (unsigned)lp.npixPad);
-    } else {
-      sLocal = (int)(id / (unsigned long long)lp.npixPad);
-      rem = (int)(id - (unsigned long long)sLocal * lp.npixPad);
-    }
-    int tile = rem >> 6, within = rem & 63;
+    int tile = rem >> 6;
     int tx = tile % lp.tilesX, ty = tile / lp.tilesX;
-    px = tx * 8 + (within & 7);
-    py = ty * 8 + (within >> 3);
+    px = tx * 8 + tileX(within);
+    py = ty * 8 + tileY(within);
   }
   if (px >= lp.width || py >= lp.height) return false;
   startPathAt(lp, px, py, lp.sampleOffset + sLocal, p);
-  p.slot = sLocal * (lp.width * lp.height) + py * lp.width + px;
+  p.slot = (py * lp.width + px) * lp.sppThisLaunch + sLocal;
   return true;
 }
 

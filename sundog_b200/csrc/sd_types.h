@@ -203,13 +203,13 @@ struct SdLaunch {
   int transparentShadows;
   int aovOn;
 
-  // work decomposition: path p -> (sample p / npixPad, tile-ordered pixel)
+  // work decomposition: path p -> (tile-ordered pixel p / sppThisLaunch, sample)
   int tilesX;
   int npixPad;
   // Tile shard (one GPU of several): shardCount > 1 renders only the 64x64
   // film tiles t (row-major over shardTilesX tiles across) with
-  // t % shardCount == shardIndex; path p -> (sample p / shardPad, owned tile,
-  // 8x8 block, pixel). Every pixel keeps the seeds of the whole-frame render.
+  // t % shardCount == shardIndex; path p -> (owned tile, 8x8 block, pixel,
+  // sample). Every pixel keeps the seeds of the whole-frame render.
   int shardCount;
   int shardIndex;
   int shardTilesX;
@@ -218,9 +218,9 @@ struct SdLaunch {
   unsigned long long* pathCounter;
   unsigned long long* rayCounter;
 
-  float4* sampleL;       // [sppThisLaunch][npixPad] radiance per sample
-  float4* sampleAlb;     // [sppThisLaunch][npixPad] first-hit albedo
-  float4* sampleNrm;     // [sppThisLaunch][npixPad] first-hit normal (camera)
+  float4* sampleL;       // [pixel][sppThisLaunch] radiance per sample
+  float4* sampleAlb;     // [pixel][sppThisLaunch] first-hit albedo
+  float4* sampleNrm;     // [pixel][sppThisLaunch] first-hit normal (camera)
   float4* accum;         // film running means [height*width]
   float4* aovAlbedo;
   float4* aovNormal;

@@ -3,8 +3,8 @@
 // A batch is a list of tile-passes (job slot, pixel rectangle, sample
 // range). Path ids run over the batch: item i owns ids [pathBegin_i,
 // pathBegin_i + npad_i * sampleCount_i), with the item's pixels in 8x8 blocks
-// (npad_i = the rectangle rounded up to whole blocks) so a warp starts on an
-// 8x4 patch of neighbouring camera rays. The kernel keeps the path tracer's
+// (npad_i = the rectangle rounded up to whole blocks) and the samples of a
+// pixel consecutive, so a warp starts on one pixel's camera rays. The kernel keeps the path tracer's
 // lane refill (ptPersistent): a lane whose path ends takes the next id,
 // whatever job it belongs to, so jobs share warps and the launch stays full
 // until the batch runs dry. A lane reads its job's launch block from the
@@ -33,11 +33,10 @@ __device__ __forceinline__ bool serveStart(unsigned long long id, Path& p, int& 
     else hi = mid - 1;
   }
   const ServeItem& it = b.items[lo];
-  unsigned long long local = id - it.pathBegin;
-  int sLocal = (int)(local / (unsigned long long)it.npad);
-  int rem = (int)(local - (unsigned long long)sLocal * it.npad);
+  int rem, sLocal;
+  splitPathId(id - it.pathBegin, it.sampleCount, rem, sLocal);
   int blk = rem >> 6, within = rem & 63;
-  int lx = (blk % it.bw) * 8 + (within & 7), ly = (blk / it.bw) * 8 + (within >> 3);
+  int lx = (blk % it.bw) * 8 + tileX(within), ly = (blk / it.bw) * 8 + tileY(within);
   if (lx >= it.w || ly >= it.h) return false;
   job = it.job;
   startPathAt(c_jobs[job], it.x0 + lx, it.y0 + ly, it.sampleBegin + sLocal, p);
@@ -100,11 +99,11 @@ __global__ void ptServeFold() {
   const int npt = it.w * it.h;
   for (int q = threadIdx.x; q < npt; q += blockDim.x) {
     int lx = q % it.w, ly = q / it.w;
-    int rem = ((ly >> 3) * it.bw + (lx >> 3)) * 64 + (ly & 7) * 8 + (lx & 7);
+    int rem = ((ly >> 3) * it.bw + (lx >> 3)) * 64 + tileIndex(lx & 7, ly & 7);
     size_t pix = (size_t)(it.y0 + ly) * lp.width + it.x0 + lx;
     float4 acc = lp.accum[pix];
     for (int k = 0; k < it.sampleCount; k++) {
-      float4 x = b.sampleL[it.pathBegin + (unsigned long long)k * it.npad + rem];
+      float4 x = b.sampleL[it.pathBegin + (unsigned long long)rem * it.sampleCount + k];
       int s1 = it.sampleBegin + k + 1;
       acc = make_float4(acc.x + (x.x - acc.x) / s1, acc.y + (x.y - acc.y) / s1,
                         acc.z + (x.z - acc.z) / s1, 1.0f);

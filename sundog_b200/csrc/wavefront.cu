@@ -103,11 +103,10 @@ __device__ __forceinline__ bool serveStartW(unsigned long long id, Path& p, int&
     else hi = mid - 1;
   }
   const ServeItem& it = b.items[lo];
-  unsigned long long local = id - it.pathBegin;
-  int sLocal = (int)(local / (unsigned long long)it.npad);
-  int rem = (int)(local - (unsigned long long)sLocal * it.npad);
+  int rem, sLocal;
+  splitPathId(id - it.pathBegin, it.sampleCount, rem, sLocal);
   int blk = rem >> 6, within = rem & 63;
-  int lx = (blk % it.bw) * 8 + (within & 7), ly = (blk / it.bw) * 8 + (within >> 3);
+  int lx = (blk % it.bw) * 8 + tileX(within), ly = (blk / it.bw) * 8 + tileY(within);
   if (lx >= it.w || ly >= it.h) return false;
   job = it.job;
   startPathAt(c_wjobs[job], it.x0 + lx, it.y0 + ly, it.sampleBegin + sLocal, p);
