@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kRenderBlock) ptTileNoAlloc() {
     Path p;
     if (!startPath(lp, fullFrameId(lp, px, py, sLocal), p)) continue;
     p.slot = (int)i;
-    while (bounce<false>(lp, p, rays, nullptr)) {
+    while (bounce<false, 0, kRoundTile>(lp, p, rays, nullptr)) {
     }
     float3 L = sanitize3(p.L);
     lp.sampleL[i] = make_float4(L.x, L.y, L.z, 1.0f);
@@ -179,6 +179,7 @@ extern "C" int sundog_session_render_tile_noalloc(sundog_session* sh, int x0, in
   const int first = s.sampleBase + sample_begin;
   SdLaunch lp = s.lp;
   lp.shardCount = 0;  // ids below use the whole-frame numbering
+  lp.sampleMajor = 0;
   lp.aovOn = 0;
   lp.sampleOffset = first;
   lp.sppThisLaunch = sample_count;

@@ -48,8 +48,6 @@ struct Path {
   unsigned long long med;  // medium stack: 4 x 16-bit material ids
   int medDepth;
   int depth;
-  int pixel;
-  int s;
   int slot;
   bool specular;
 };
@@ -63,8 +61,6 @@ __device__ __forceinline__ uint16_t medAt(unsigned long long med, int i) {
 // only on (pixel, s, seed). (device/programs.cu:312-357)
 __device__ __forceinline__ void startPathAt(const SdLaunch& lp, int px, int py, int s, Path& p) {
   int pixel = py * lp.width + px;
-  p.pixel = pixel;
-  p.s = s;
   p.rng = Pcg::seeded(((unsigned long long)pixel << 32) ^ (unsigned long long)s,
                       (unsigned long long)lp.seed);
   int ns = lp.nStrata;
@@ -107,25 +103,28 @@ __device__ __forceinline__ int tileIndex(int x, int y) {
          ((y & 4) << 3);
 }
 
-// Splits a path index into (tile-ordered pixel, sample of `spp`): the samples
-// of a pixel are consecutive, so a warp holds the samples of one pixel (or of
-// a small patch when spp < 32) and its camera rays visit the same nodes,
-// textures and materials.
-__device__ __forceinline__ void splitPathId(unsigned long long id, int spp, int& pixel, int& s) {
+// Splits a path index by its inner extent: (tile-ordered pixel, sample of
+// `inner`). The samples of a pixel are consecutive, so a warp holds the
+// samples of one pixel (or of a small patch when there are fewer than 32) and
+// its camera rays visit the same nodes, textures and materials.
+__device__ __forceinline__ void splitPathId(unsigned long long id, int inner, int& q, int& r) {
   if (id < (1ull << 32)) {  // a 32-bit division: the common case, far cheaper
     const unsigned id32 = (unsigned)id;
-    pixel = (int)(id32 / (unsigned)spp);
-    s = (int)(id32 - (unsigned)pixel * (unsigned)spp);
+    q = (int)(id32 / (unsigned)inner);
+    r = (int)(id32 - (unsigned)q * (unsigned)inner);
   } else {
-    pixel = (int)(id / (unsigned long long)spp);
-    s = (int)(id - (unsigned long long)pixel * spp);
+    q = (int)(id / (unsigned long long)inner);
+    r = (int)(id - (unsigned long long)q * inner);
   }
 }
 
-// Camera sample for path index id; false if the index is tile padding.
-__device__ __forceinline__ bool startPath(const SdLaunch& lp, unsigned long long id, Path& p) {
-  int rem, sLocal, px, py;
-  splitPathId(id, lp.sppThisLaunch, rem, sLocal);
+// Pixel and launch-local sample of path index id; false if the index is tile
+// padding.
+__device__ __forceinline__ bool pathPixel(const SdLaunch& lp, unsigned long long id, int& px,
+                                          int& py, int& sLocal) {
+  int rem;
+  if (lp.sampleMajor) splitPathId(id, lp.shardCount > 1 ? lp.shardPad : lp.npixPad, sLocal, rem);
+  else splitPathId(id, lp.sppThisLaunch, rem, sLocal);
   const int within = rem & 63;
   if (lp.shardCount > 1) {
     int tile = (rem >> 12) * lp.shardCount + lp.shardIndex;
@@ -138,9 +137,20 @@ __device__ __forceinline__ bool startPath(const SdLaunch& lp, unsigned long long
     px = tx * 8 + tileX(within);
     py = ty * 8 + tileY(within);
   }
-  if (px >= lp.width || py >= lp.height) return false;
+  return px < lp.width && py < lp.height;
+}
+
+// A sample's place in the launch's per-sample buffers.
+__device__ __forceinline__ int sampleSlot(const SdLaunch& lp, int px, int py, int sLocal) {
+  return (py * lp.width + px) * lp.sppThisLaunch + sLocal;
+}
+
+// Camera sample for path index id; false if the index is tile padding.
+__device__ __forceinline__ bool startPath(const SdLaunch& lp, unsigned long long id, Path& p) {
+  int px, py, sLocal;
+  if (!pathPixel(lp, id, px, py, sLocal)) return false;
   startPathAt(lp, px, py, lp.sampleOffset + sLocal, p);
-  p.slot = (py * lp.width + px) * lp.sppThisLaunch + sLocal;
+  p.slot = sampleSlot(lp, px, py, sLocal);
   return true;
 }
 
@@ -169,29 +179,33 @@ struct Vertex {
   bool delta;
 };
 
-// First half of a path segment, after its radiance ray was traced (hit,
-// h): media, flames, escape, surface shading, emission, and the NEE light
-// draw. Returns false when the path has ended; otherwise v holds the vertex
-// and, if v.nee, the shadow ray to trace. (device/programs.cu:374-495)
-template <bool COUNT>
-__device__ __forceinline__ bool shadeVertex(const SdLaunch& lp, Path& p, bool hit,
-                                            const TraceHit& h, unsigned long long& rays,
-                                            Vertex& v) {
-  const bool hasEnv = lp.bgKind == BG_ENVMAP;
-  const int nStrat = lp.numLights + (hasEnv ? 1 : 0);
-
+// The traced segment's media: absorption of the medium the path is in, then
+// the flames along the segment. t: the hit's distance.
+// (device/programs.cu:374-400)
+__device__ __forceinline__ void crossMedia(const SdLaunch& lp, Path& p, bool hit, float t) {
   if (p.medDepth > 0) {
     int top = min(p.medDepth, 4) - 1;
     float3 sigma = lp.materials[medAt(p.med, top)].absorb;
-    if (hmax(sigma) > 0.0f) p.beta *= vexp(-sigma * (hit ? h.t : 1e4f));
+    if (hmax(sigma) > 0.0f) p.beta *= vexp(-sigma * (hit ? t : 1e4f));
   }
 
   if (lp.numFlames > 0) {
     float3 trans = v3(1.0f);
-    float3 Lv = flameMarch(lp.flames, lp.numFlames, p.o, p.d, hit ? h.t : 1e16f, p.rng, trans);
+    float3 Lv = flameMarch(lp.flames, lp.numFlames, p.o, p.d, hit ? t : 1e16f, p.rng, trans);
     addClamped(lp, p, p.beta * Lv);
     p.beta *= trans;
   }
+}
+
+// First half of a path segment after its media: escape, surface shading,
+// emission, and the NEE light draw. Returns false when the path has ended;
+// otherwise v holds the vertex and, if v.nee, the shadow ray to trace.
+// (device/programs.cu:400-495)
+__device__ __forceinline__ bool shadeSurface(const SdLaunch& lp, Path& p, bool hit,
+                                             const TraceHit& h, unsigned long long& rays,
+                                             Vertex& v) {
+  const bool hasEnv = lp.bgKind == BG_ENVMAP;
+  const int nStrat = lp.numLights + (hasEnv ? 1 : 0);
 
   if (!hit) {
     float3 bg = background(lp, p.d);
@@ -274,38 +288,37 @@ __device__ __forceinline__ bool shadeVertex(const SdLaunch& lp, Path& p, bool hi
   return true;
 }
 
-// Second half of a path segment: the NEE contribution given the shadow
-// ray's transmittance tr, the BSDF sample, the medium stack and Russian
+// The NEE contribution of v before its shadow ray's transmittance.
+__device__ __forceinline__ float3 neeTerm(const SdLaunch& lp, const Path& p, const SdMaterial& mat,
+                                          const Vertex& v) {
+  const int nStrat = lp.numLights + (lp.bgKind == BG_ENVMAP ? 1 : 0);
+  float pdfLe = (v.delta ? 1.0f : v.pdf) / nStrat;
+  float3 f = bsdfValue(mat, v.albedo, -p.d, v.wi, v.ns, v.etaRel);
+  float w = 1.0f;
+  if (!v.delta) {
+    float pdfB = bsdfDensity(mat, -p.d, v.wi, v.ns, v.etaRel);
+    w = pdfLe / (pdfLe + pdfB);
+  }
+  return p.beta * f * fabsf(v.cosS) * v.Li * w / pdfLe;
+}
+
+// The radiance added by an NEE term c behind transmittance tr (clamped past
+// the first vertex).
+__device__ __forceinline__ float3 neeRadiance(float3 c, float3 tr, bool indirect, float clampVal) {
+  c = c * tr;
+  if (indirect && clampVal > 0.0f) c = vmin(c, v3(clampVal));
+  return sanitize3(c);
+}
+
+// The end of a path segment: the BSDF sample, the medium stack and Russian
 // roulette. Returns false when the path has ended. GUIDE selects the guided
 // variants (kGuideSample: draw by MIS with the guide; kGuideRecord: keep
-// training vertices in *trail); 0 is the reference's sampler.
-// (device/programs.cu:495-558)
-template <int GUIDE = 0>
-__device__ __forceinline__ bool finishVertex(const SdLaunch& lp, Path& p, const Vertex& v,
-                                             float3 tr, GuideTrail* trail = nullptr) {
-  const bool hasEnv = lp.bgKind == BG_ENVMAP;
-  const int nStrat = lp.numLights + (hasEnv ? 1 : 0);
-  const SdMaterial mat = lp.materials[v.matId];
+// training vertices in *trail); 0 is the reference's sampler. ROUND: the
+// kernel's Rounding. (device/programs.cu:520-558)
+template <int GUIDE, int ROUND>
+__device__ __forceinline__ bool sampleNext(const SdLaunch& lp, Path& p, const SdMaterial& mat,
+                                           const Vertex& v, GuideTrail* trail) {
   const float3 x = v.x, ns = v.ns, albedo = v.albedo;
-
-  if (v.nee && hmax(tr) > 0.0f) {
-    if (lp.numFlames > 0 && lp.transparentShadows) {
-      int skip = v.lightK < lp.numLights ? lp.lights[v.lightK].flameId : -1;
-      tr = tr * flameShadow(lp.flames, lp.numFlames, v.so, v.wi, v.tmaxS, p.rng, skip);
-    }
-    float pdfLe = (v.delta ? 1.0f : v.pdf) / nStrat;
-    float3 f = bsdfValue(mat, albedo, -p.d, v.wi, ns, v.etaRel);
-    float w = 1.0f;
-    if (!v.delta) {
-      float pdfB = bsdfDensity(mat, -p.d, v.wi, ns, v.etaRel);
-      w = pdfLe / (pdfLe + pdfB);
-    }
-    float3 c = p.beta * f * fabsf(v.cosS) * v.Li * w / pdfLe;
-    c = c * tr;
-    if (p.depth >= 1 && lp.clampVal > 0.0f) c = vmin(c, v3(lp.clampVal));
-    p.L += sanitize3(c);
-  }
-
   BsdfDraw bs;
   float pdfSample;  // density wi was drawn with (differs from bs.pdf when guided)
   if ((GUIDE & kGuideSample) && guideEligible(mat)) {
@@ -313,7 +326,7 @@ __device__ __forceinline__ bool finishVertex(const SdLaunch& lp, Path& p, const 
     bs = gd.s;
     pdfSample = gd.pdfSample;
   } else {
-    bs = bsdfDraw(mat, albedo, p.d, ns, v.front, v.etaExt, p.rng);
+    bs = bsdfDraw<ROUND>(mat, albedo, p.d, ns, v.front, v.etaExt, p.rng);
     pdfSample = bs.pdf;
   }
   if (!bs.ok) return false;
@@ -348,14 +361,30 @@ __device__ __forceinline__ bool finishVertex(const SdLaunch& lp, Path& p, const 
   return p.depth < lp.maxDepth;
 }
 
+// Second half of a path segment: the NEE contribution given the shadow
+// ray's transmittance tr, then sampleNext. (device/programs.cu:495-558)
+template <int GUIDE, int ROUND>
+__device__ __forceinline__ bool finishVertex(const SdLaunch& lp, Path& p, const Vertex& v,
+                                             float3 tr, GuideTrail* trail = nullptr) {
+  const SdMaterial mat = lp.materials[v.matId];
+  if (v.nee && hmax(tr) > 0.0f) {
+    if (lp.numFlames > 0 && lp.transparentShadows) {
+      int skip = v.lightK < lp.numLights ? lp.lights[v.lightK].flameId : -1;
+      tr = tr * flameShadow(lp.flames, lp.numFlames, v.so, v.wi, v.tmaxS, p.rng, skip);
+    }
+    p.L += neeRadiance(neeTerm(lp, p, mat, v), tr, p.depth >= 1, lp.clampVal);
+  }
+  return sampleNext<GUIDE, ROUND>(lp, p, mat, v, trail);
+}
+
 // One segment of the path for the persistent kernels: the radiance ray,
-// shadeVertex, the shadow ray and finishVertex -- the same functions the
+// crossMedia, shadeSurface, the shadow ray and finishVertex -- the functions the
 // wavefront stages call, in the same order with the same random draws, so
 // both engines trace the same samples. Returns false when the path has
 // ended. GUIDE selects the guided variants (kGuideSample: draw by MIS with
 // the guide; kGuideRecord: keep training vertices in *trail); 0 is the
 // reference's sampler. (device/programs.cu:374-558)
-template <bool COUNT, int GUIDE = 0>
+template <bool COUNT, int GUIDE = 0, int ROUND = kRoundFree>
 __device__ __forceinline__ bool bounce(const SdLaunch& lp, Path& p, unsigned long long& rays,
                                        TraceCount* cnt, GuideTrail* trail = nullptr) {
   TraceHit h;
@@ -364,11 +393,12 @@ __device__ __forceinline__ bool bounce(const SdLaunch& lp, Path& p, unsigned lon
   const bool hit = traverse<false, COUNT>(lp, p.o, p.d, 1e16f, h, dummyTr, dummyTau, cnt);
   rays++;
   Vertex v;
-  if (!shadeVertex<COUNT>(lp, p, hit, h, rays, v)) return false;
+  crossMedia(lp, p, hit, h.t);
+  if (!shadeSurface(lp, p, hit, h, rays, v)) return false;
   float3 tr = v3(0.0f);
   // Counting build: shadow traversals go to the second counter set.
   if (v.nee) tr = shadowTransmittance<COUNT>(lp, v.so, v.wi, v.tmaxS, COUNT ? cnt + 1 : nullptr);
-  return finishVertex<GUIDE>(lp, p, v, tr, trail);
+  return finishVertex<GUIDE, ROUND>(lp, p, v, tr, trail);
 }
 
 }  // namespace sdb

@@ -827,6 +827,7 @@ void RenderSession::render(cudaStream_t st, bool reset, sundog_render_result* re
     }
     lp.sampleOffset = sampleBase + done;
     lp.sppThisLaunch = n;
+    lp.sampleMajor = (mode & kGuideRecord) ? 1 : 0;
     lp.numPaths = (unsigned long long)pathsPerSample(lp) * n;
     cudaCheck(cudaMemsetAsync(lp.pathCounter, 0, sizeof(unsigned long long), st), "counter reset");
     {
@@ -841,7 +842,8 @@ void RenderSession::render(cudaStream_t st, bool reset, sundog_render_result* re
         // A tile shard that owns no tile: nothing to trace.
       } else if (wavefront) {
         if (!wf) wf = wfAcquire();
-        wf->ensure((int)std::min<unsigned long long>(lp.numPaths, kWavefrontSlots));
+        wf->ensure((int)std::min<unsigned long long>(lp.numPaths, kWavefrontSlots),
+                   wfHasLate(lp, mode));
         launches += wfRender(lp, *wf, st, mode, stageTiming ? &stages : nullptr);
       } else {
         cudaCheck(launchRender(st, grid, mode), "path kernel launch");
@@ -897,6 +899,7 @@ void RenderSession::countTraversal(sundog_trace_counts* out, sundog_trace_counts
     int n = std::min(chunk, lp.sppTotal - done);
     lp.sampleOffset = sampleBase + done;
     lp.sppThisLaunch = n;
+    lp.sampleMajor = 0;
     lp.numPaths = (unsigned long long)pathsPerSample(lp) * n;
     cudaCheck(cudaMemsetAsync(lp.pathCounter, 0, sizeof(unsigned long long), stream), "counter reset");
     std::lock_guard<std::mutex> launchLock(deviceLaunchLock());

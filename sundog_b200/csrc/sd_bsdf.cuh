@@ -13,6 +13,112 @@
 
 namespace sdb {
 
+// Where the compiler may contract a product into a sum in more than one way,
+// what surrounds an inlined function decides, and a last bit that differs
+// sends a refracted path elsewhere. The kernels that must go on drawing the
+// samples they always drew name their form of the refraction instead:
+//   kRoundFree   left to the compiler (the persistent megakernel)
+//   kRoundStage  the wavefront stages: smooth interfaces with a rounded
+//                cos^2, rough ones with a fused cos^2, and the order of every
+//                sum of products
+//   kRoundServe  the stages of a serving batch: every cos^2 fused
+//   kRoundTile   the allocation-free tile render: rough ones as the stages
+enum Rounding : int { kRoundFree = 0, kRoundStage, kRoundServe, kRoundTile };
+
+#if defined(__CUDA_ARCH__)
+__device__ __forceinline__ float3 unitXyz(float3 a) {
+  const float r = 1.0f / sqrtf(__fmaf_rn(a.z, a.z, __fmaf_rn(a.y, a.y, __fmul_rn(a.x, a.x))));
+  return v3(__fmul_rn(a.x, r), __fmul_rn(a.y, r), __fmul_rn(a.z, r));
+}
+__device__ __forceinline__ float3 mirrorUnitXyz(float3 v, float3 n) {
+  const float m =
+      -2.0f * __fmaf_rn(v.z, n.z, __fmaf_rn(v.x, n.x, __fmul_rn(v.y, n.y)));
+  return unitXyz(v3(__fmaf_rn(m, n.x, v.x), __fmaf_rn(m, n.y, v.y), __fmaf_rn(m, n.z, v.z)));
+}
+// snell with every rounding named. C2: cos^2 rounded before it is subtracted
+// (else fused); INCIDENT: the direction's sum folded from the incident side
+// (else from the normal's).
+template <bool C2, bool INCIDENT>
+__device__ __forceinline__ bool snellRounded(float3 v, float3 n, float eta, float3& t) {
+  const float ci =
+      INCIDENT ? -__fmaf_rn(v.z, n.z, __fmaf_rn(v.x, n.x, __fmul_rn(v.y, n.y)))
+               : -__fmaf_rn(v.z, n.z, __fmaf_rn(v.y, n.y, __fmul_rn(v.x, n.x)));
+  const float q = C2 ? __fsub_rn(1.0f, __fmul_rn(ci, ci)) : __fmaf_rn(-ci, ci, 1.0f);
+  const float k = __fmaf_rn(-__fmul_rn(eta, eta), q, 1.0f);
+  if (k < 0.0f) return false;
+  const float a = __fsub_rn(__fmul_rn(eta, ci), sqrtf(k));
+  if (INCIDENT)
+    t = v3(__fmaf_rn(eta, v.x, __fmul_rn(a, n.x)), __fmaf_rn(eta, v.y, __fmul_rn(a, n.y)),
+           __fmaf_rn(eta, v.z, __fmul_rn(a, n.z)));
+  else
+    t = v3(__fmaf_rn(a, n.x, __fmul_rn(eta, v.x)), __fmaf_rn(a, n.y, __fmul_rn(eta, v.y)),
+           __fmaf_rn(a, n.z, __fmul_rn(eta, v.z)));
+  return true;
+}
+#endif
+
+// The refraction, reflection and refracted direction of a smooth interface,
+// and the refraction of a rough one, in a kernel's form.
+template <int ROUND>
+SDB_HD bool snellSmooth(float3 v, float3 n, float eta, float3& t) {
+#if defined(__CUDA_ARCH__)
+  if (ROUND == kRoundStage) return snellRounded<true, true>(v, n, eta, t);
+  if (ROUND == kRoundServe) return snellRounded<false, true>(v, n, eta, t);
+#endif
+  return snell(v, n, eta, t);
+}
+template <int ROUND>
+SDB_HD bool snellRough(float3 v, float3 n, float eta, float3& t) {
+#if defined(__CUDA_ARCH__)
+  if (ROUND != kRoundFree) return snellRounded<false, false>(v, n, eta, t);
+#endif
+  return snell(v, n, eta, t);
+}
+template <int ROUND>
+SDB_HD float3 mirrorRough(float3 v, float3 n) {
+#if defined(__CUDA_ARCH__)
+  if (ROUND != kRoundFree) {
+    const float m = -2.0f * __fmaf_rn(v.z, n.z, __fmaf_rn(v.y, n.y, __fmul_rn(v.x, n.x)));
+    return v3(__fmaf_rn(m, n.x, v.x), __fmaf_rn(m, n.y, v.y), __fmaf_rn(m, n.z, v.z));
+  }
+#endif
+  return mirror(v, n);
+}
+template <int ROUND>
+SDB_HD float3 unitRough(float3 a) {
+#if defined(__CUDA_ARCH__)
+  if (ROUND != kRoundFree) {
+    const float r = 1.0f / sqrtf(__fmaf_rn(a.z, a.z, __fmaf_rn(a.x, a.x, __fmul_rn(a.y, a.y))));
+    return v3(__fmul_rn(a.x, r), __fmul_rn(a.y, r), __fmul_rn(a.z, r));
+  }
+#endif
+  return unit(a);
+}
+template <int ROUND>
+SDB_HD float3 toWorldRough(const Frame& f, float3 v) {
+#if defined(__CUDA_ARCH__)
+  if (ROUND != kRoundFree)
+    return v3(__fmaf_rn(v.z, f.n.x, __fmaf_rn(v.x, f.t.x, __fmul_rn(v.y, f.b.x))),
+              __fmaf_rn(v.z, f.n.y, __fmaf_rn(v.x, f.t.y, __fmul_rn(v.y, f.b.y))),
+              __fmaf_rn(v.z, f.n.z, __fmaf_rn(v.x, f.t.z, __fmul_rn(v.y, f.b.z))));
+#endif
+  return f.toWorld(v);
+}
+template <int ROUND>
+SDB_HD float3 reflectSmooth(float3 v, float3 n) {
+#if defined(__CUDA_ARCH__)
+  if (ROUND == kRoundStage || ROUND == kRoundServe) return mirrorUnitXyz(v, n);
+#endif
+  return unit(mirror(v, n));
+}
+template <int ROUND>
+SDB_HD float3 unitSmooth(float3 v) {
+#if defined(__CUDA_ARCH__)
+  if (ROUND == kRoundStage || ROUND == kRoundServe) return unitXyz(v);
+#endif
+  return unit(v);
+}
+
 struct BsdfDraw {
   float3 wi;
   float3 weight;  // f |cos| / pdf, or the delta weight
@@ -224,6 +330,7 @@ SDB_HD float bsdfDensity(const SdMaterial& m, float3 wo, float3 wi, float3 n, fl
 // Draws: lambert 2; metal 0 (mirror) / 2; smooth glass & water 1 when
 // refraction is possible, 0 on TIR; rough glass 2 + 1 unless the facet
 // reflects totally; plastic exactly 3. (device/bsdf.cuh:271-424)
+template <int ROUND = kRoundFree>
 SDB_HD BsdfDraw bsdfDraw(const SdMaterial& m, float3 albedo, float3 d, float3 n,
                          bool frontface, float etaExt, Pcg& rng) {
   BsdfDraw s;
@@ -275,15 +382,15 @@ SDB_HD BsdfDraw bsdfDraw(const SdMaterial& m, float3 albedo, float3 d, float3 n,
       f0 = f0 * f0;
       if (m.kind == MT_WATER || m.roughness < 1e-3f) {
         s.delta = true;
-        if (snell(d, n, eta, refr)) {
+        if (snellSmooth<ROUND>(d, n, eta, refr)) {
           float c = eta < 1.0f ? -dot(d, n) : -dot(refr, n);
           float pr = fresnelSchlick(c, f0);
           if (rng.uni() < pr)
-            s.wi = unit(mirror(d, n));
+            s.wi = reflectSmooth<ROUND>(d, n);
           else
-            s.wi = unit(refr);
+            s.wi = unitSmooth<ROUND>(refr);
         } else {
-          s.wi = unit(mirror(d, n));
+          s.wi = reflectSmooth<ROUND>(d, n);
         }
         s.weight = v3(1.0f);
         s.ok = true;
@@ -297,24 +404,24 @@ SDB_HD BsdfDraw bsdfDraw(const SdMaterial& m, float3 albedo, float3 d, float3 n,
       float loh = dot(lo, h);
       if (loh <= 0.0f) return s;
       float3 li;
-      if (!snell(-lo, h, eta, refr)) {
-        li = mirror(-lo, h);
+      if (!snellRough<ROUND>(-lo, h, eta, refr)) {
+        li = mirrorRough<ROUND>(-lo, h);
         if (li.z <= 0.0f) return s;
         s.pdf = ggxPdfReflect(lo, li, a);
       } else {
         float c = eta < 1.0f ? loh : -dot(refr, h);
         float pr = fresnelSchlick(c, f0);
         if (rng.uni() < pr) {
-          li = mirror(-lo, h);
+          li = mirrorRough<ROUND>(-lo, h);
           if (li.z <= 0.0f) return s;
           s.pdf = pr * ggxPdfReflect(lo, li, a);
         } else {
-          li = unit(refr);
+          li = unitRough<ROUND>(refr);
           if (li.z >= 0.0f) return s;
           s.pdf = (1.0f - pr) * ggxPdfTransmit(lo, li, h, eta, a);
         }
       }
-      s.wi = fr.toWorld(li);
+      s.wi = toWorldRough<ROUND>(fr, li);
       float w = ggxG(lo, li, a) / ggxG1(lo, a);
       if (li.z < 0.0f) w *= eta * eta;
       s.weight = v3(w);

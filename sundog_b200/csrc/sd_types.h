@@ -203,7 +203,11 @@ struct SdLaunch {
   int transparentShadows;
   int aovOn;
 
-  // work decomposition: path p -> (tile-ordered pixel p / sppThisLaunch, sample)
+  // work decomposition: path p -> (tile-ordered pixel p / sppThisLaunch, sample);
+  // sampleMajor: (sample, pixel) instead, for launches that keep the training
+  // records of the paths that end first (the record cap then cuts samples,
+  // not a part of the image)
+  int sampleMajor;
   int tilesX;
   int npixPad;
   // Tile shard (one GPU of several): shardCount > 1 renders only the 64x64

@@ -113,7 +113,7 @@ class Server {
     if (cfg.engine != 1) {  // the wavefront engine's slot pool, sized for a batch
       wf = wfAcquire();
       uint64_t batchPaths = cfg.iteration_paths + (uint64_t)kMaxServeJobs * maxItemPaths;
-      wf->ensure((int)std::min<uint64_t>(batchPaths, 1ull << 26));
+      wf->ensure((int)std::min<uint64_t>(batchPaths, 1ull << 26), true);
     }
     slots.assign(kMaxServeJobs, nullptr);
     thread = std::thread([this] { loop(); });
@@ -543,12 +543,8 @@ class Server {
     std::lock_guard<std::mutex> launchLock(deviceLaunchLock());
     std::vector<SdLaunch> table(kMaxServeJobs);
     std::memset(table.data(), 0, table.size() * sizeof(SdLaunch));
-    int maxInstances = 0;
     for (size_t k = 0; k < slots.size(); k++)
-      if (slots[k]) {
-        table[k] = slots[k]->lp;
-        maxInstances = std::max(maxInstances, slots[k]->lp.numInstances);
-      }
+      if (slots[k]) table[k] = slots[k]->lp;
     // Both engines fold through ptServeFold, which reads the megakernel's
     // table; the wavefront stages read their own.
     cudaCheck(serveSetJobs(table.data(), st), "job table");
@@ -566,7 +562,7 @@ class Server {
     b.sampleL = (float4*)scratch.ptr;
     cudaCheck(cudaEventRecord(ev0, st), "event");
     if (wf) {
-      wfRenderBatch(b, *wf, st, maxInstances);
+      wfRenderBatch(b, *wf, st, table.data());
       cudaCheck(serveFold(b, st), "serve fold");
     } else {
       cudaCheck(serveLaunch(b, grid, st), "serve launch");

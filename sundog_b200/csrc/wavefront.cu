@@ -1,25 +1,27 @@
 // Wavefront path tracer: the plain path kernel's per-path computation split
 // into stages over a pool of path slots held in global memory.
 //
-//   wfStart        fill every slot with a camera path
-//   per iteration, over the slots in the live list:
+//   wfStart        a camera ray in every slot
+//   per iteration (path depth), over the slots in the live list:
 //   wfTraceFetch   trace the radiance ray (traversal only)
-//   wfShadeA       shadeVertex: media, flames, escape, shading, emission, the
-//                  NEE light draw; queues the slot's shadow ray
-//   wfShadow       trace the queued shadow rays (transparent shadows)
-//   wfShadeB       finishVertex: NEE contribution, BSDF sample, roulette
+//   wfShade        media, flames, escape, shading, emission, the NEE light
+//                  draw, the BSDF sample and roulette; queues the slot's
+//                  shadow ray with the radiance it would add
+//   wfShadow       trace the queued shadow rays (transparent shadows) and
+//                  add that radiance
+//   wfLate         the end of the few vertices that must know their shadow
+//                  ray's result before they go on
 //
-// A slot whose path ends writes that sample and takes the next camera path at
-// once (warp-aggregated counter), so the pool stays full until the frame's
-// paths run out. Each stage's code is small next to the megakernel's and
-// keeps its state in registers instead of a 1 KB spilled frame, so at full
-// occupancy the instruction and local-memory traffic of the megakernel
-// disappear; the price is the path state's round trip through global memory
-// between stages (a few hundred bytes per path segment).
+// All paths of a pool are at the same depth, so the iterations of a pool are
+// known to end with the deepest path and are launched in groups without a
+// look at the live count. Each stage's code is small next to the
+// megakernel's and keeps its state in registers instead of a 1 KB spilled
+// frame; the price is the path state's round trip through global memory
+// between stages (about 200 bytes per path segment).
 //
-// The stages call the megakernel's own shadeVertex / finishVertex /
-// traverse in the same order with the same random draws, so every sample is
-// the same sample as in ptPersistent, and the film fold is unchanged.
+// The stages call the megakernel's own per-path functions in the same order
+// with the same random draws, so every sample is the same sample as in
+// ptPersistent, and the film fold is unchanged.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -55,25 +57,38 @@ __device__ __forceinline__ const SdLaunch& slotLaunch(int slot) {
   return c_wlp;
 }
 
+template <int GUIDE>
+constexpr int kRound = (GUIDE & kWfServe) ? kRoundServe : kRoundStage;  // sd_bsdf.cuh
+
 #ifndef SDB_WF_TRACE_BLOCKS
 #define SDB_WF_TRACE_BLOCKS 8
 #endif
 // Resident blocks per SM the stage kernels are compiled for: traversal 8 ->
-// 64 registers, shading 5 -> 102 registers. Shading at 6 blocks (80
-// registers) gains on config 1 and 2 (1,716 / 2,558 against 1,697 / 2,507
-// Mrays/s) and loses on config 0 and the gallery scenes, whose shading
-// spills more at 80 registers (01-marble-run 4,476 against 4,709,
-// 02-cornell-lume 3,673 against 3,819); 4 blocks lose on all (1,648 /
-// 2,402 on configs 1 / 2).
+// 64 registers, shading 5 -> 102 registers.
 #ifndef SDB_WF_SHADE_BLOCKS
 #define SDB_WF_SHADE_BLOCKS 5
 #endif
-// The second shading stage alone at 6 blocks (80 registers): config 1
-// 1,718 -> 1,729 Mrays/s, config 0 2,756 -> 2,779, config 2 and the gallery
-// scenes within 0.2%.
-#ifndef SDB_WF_SHADEB_BLOCKS
-#define SDB_WF_SHADEB_BLOCKS 6
-#endif
+
+// A 32-byte record in one 256-bit load or store.
+struct Rec {
+  float4 a, b;
+};
+__device__ __forceinline__ Rec ldRec(const float4* p, int slot) {
+  Rec r;
+  asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y),
+                 "=f"(r.b.z), "=f"(r.b.w)
+               : "l"(p + 2 * (size_t)slot)
+               : "memory");
+  return r;
+}
+__device__ __forceinline__ void stRec(float4* p, int slot, float4 a, float4 b) {
+  asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p + 2 * (size_t)slot),
+               "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+               : "memory");
+}
+__device__ __forceinline__ float bitsF(unsigned v) { return __uint_as_float(v); }
+__device__ __forceinline__ unsigned bitsU(float v) { return __float_as_uint(v); }
 
 // Slot index for an append to a list by the calling lanes together.
 __device__ __forceinline__ unsigned appendSlot(unsigned* count) {
@@ -83,18 +98,10 @@ __device__ __forceinline__ unsigned appendSlot(unsigned* count) {
   return g.shfl(base, 0) + g.thread_rank();
 }
 
-template <int GUIDE>
-__device__ __forceinline__ unsigned long long nextPathId() {
-  cg::coalesced_group g = cg::coalesced_threads();
-  unsigned long long* counter = (GUIDE & kWfServe) ? c_wbatch.pathCounter : c_wlp.pathCounter;
-  unsigned long long base = 0;
-  if (g.thread_rank() == 0) base = atomicAdd(counter, (unsigned long long)g.size());
-  return g.shfl(base, 0) + g.thread_rank();
-}
-
-// Serving: path id -> its tile-pass's camera sample (false for block
+// Serving: path id -> its tile-pass's pixel and sample (false for block
 // padding), as serveStart in serve.cu.
-__device__ __forceinline__ bool serveStartW(unsigned long long id, Path& p, int& job) {
+__device__ __forceinline__ bool servePixel(unsigned long long id, int& job, int& px, int& py,
+                                           int& sample) {
   const ServeBatch& b = c_wbatch;
   int lo = 0, hi = b.numItems - 1;
   while (lo < hi) {
@@ -109,97 +116,65 @@ __device__ __forceinline__ bool serveStartW(unsigned long long id, Path& p, int&
   int lx = (blk % it.bw) * 8 + tileX(within), ly = (blk / it.bw) * 8 + tileY(within);
   if (lx >= it.w || ly >= it.h) return false;
   job = it.job;
-  startPathAt(c_wjobs[job], it.x0 + lx, it.y0 + ly, it.sampleBegin + sLocal, p);
-  p.slot = (int)id;
+  px = it.x0 + lx;
+  py = it.y0 + ly;
+  sample = it.sampleBegin + sLocal;
   return true;
 }
 
-// Puts the next camera path in `slot` and lists it in list `out`; leaves the
-// slot empty when the frame's paths are used up. Record passes (GUIDE &
-// kGuideRecord) start the slot's trail empty.
+// Hit record markers (in place of the instance).
+constexpr int kMiss = -1;
+constexpr int kNoPath = -2;  // a slot of tile padding
+
+// Camera rays into the first n slots: slot i takes path base + i. Only the
+// ray and the random state are stored (32 bytes); the rest of a fresh path
+// is constant and the first shading stage fills it in.
 template <int GUIDE>
-__device__ __forceinline__ void refill(int slot, int out, bool start = false) {
+__global__ void __launch_bounds__(kRenderBlock) wfStart(unsigned long long base, unsigned n) {
   const WfPool& pool = c_pool;
-  // When the start stage placed every path, a slot whose path ends has no id
-  // left to take: skip the atomic on the path counter that would say so.
-  if (!start && !pool.refillOpen) return;
-  const unsigned long long numPaths = (GUIDE & kWfServe) ? c_wbatch.numPaths : c_wlp.numPaths;
-  while (true) {
-    unsigned long long id = nextPathId<GUIDE>();
-    if (id >= numPaths) return;
-    Path p;
-    int job = 0;
-    if ((GUIDE & kWfServe) ? serveStartW(id, p, job) : startPath(c_wlp, id, p)) {
-      pool.paths[slot].v = p;
-      if (GUIDE & kWfServe) pool.jobs[slot] = (unsigned char)job;
-      if (GUIDE & kGuideRecord) pool.trails[slot].v.n = 0;
-      pool.lists[out][appendSlot(&pool.counts[out])] = slot;
-      return;
-    }
-  }
-}
-
-// The finished path's sample; record passes also turn its trail of guided
-// vertices into training records.
-template <int GUIDE>
-__device__ __forceinline__ void finishPath(const Path& p, int slot) {
-  float3 L = sanitize3(p.L);
-  if (GUIDE & kGuideRecord) guideFlush(c_wlp, c_pool.trails[slot].v, L);
-  float4* sampleL = (GUIDE & kWfServe) ? c_wbatch.sampleL : c_wlp.sampleL;
-  sampleL[p.slot] = make_float4(L.x, L.y, L.z, 1.0f);
-}
-
-template <int GUIDE = 0>
-__device__ __forceinline__ void addRays(unsigned long long rays) {
-  for (int off = 16; off > 0; off >>= 1) rays += __shfl_down_sync(0xFFFFFFFFu, rays, off);
-  unsigned long long* counter = (GUIDE & kWfServe) ? c_wbatch.rayCounter : c_wlp.rayCounter;
-  if ((threadIdx.x & 31) == 0 && rays) atomicAdd(counter, rays);
-}
-
-template <int GUIDE>
-__global__ void __launch_bounds__(kRenderBlock) wfStart() {
-  const WfPool& pool = c_pool;
-  for (int slot = blockIdx.x * blockDim.x + threadIdx.x; slot < pool.cap;
-       slot += gridDim.x * blockDim.x)
-    refill<GUIDE>(slot, 0, true);
-}
-
-// Camera paths into the pool without atomics, for frames whose 8x8 pixel
-// tiles cover the image exactly (every path id is a pixel sample, so
-// refill's id counter and list appends would only number the slots in
-// order): slot i takes path i, the live list is the identity, and the list
-// length and path counter continue from n = min(pool, paths). The same
-// paths in the same slots as wfStart.
-template <int GUIDE>
-__global__ void __launch_bounds__(kRenderBlock) wfStartDirect(unsigned n) {
-  const WfPool& pool = c_pool;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    pool.counts[0] = n;
-    *c_wlp.pathCounter = n;
-  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) pool.counts[0].live = n;
   for (unsigned slot = blockIdx.x * blockDim.x + threadIdx.x; slot < n;
        slot += gridDim.x * blockDim.x) {
     Path p;
-    startPath(c_wlp, slot, p);
-    pool.paths[slot].v = p;
-    if (GUIDE & kGuideRecord) pool.trails[slot].v.n = 0;
-    pool.lists[0][slot] = (int)slot;
+    bool ok;
+    if (GUIDE & kWfServe) {
+      int job = 0, px, py, s;
+      ok = servePixel(base + slot, job, px, py, s);
+      pool.jobs[slot] = (unsigned char)job;
+      if (ok) startPathAt(c_wjobs[job], px, py, s, p);
+    } else {
+      ok = startPath(c_wlp, base + slot, p);
+    }
+    if (!ok) {
+      pool.hits[2 * (size_t)slot] = make_float4(0.0f, __int_as_float(kNoPath), 0.0f, 0.0f);
+      p.o = p.d = v3(0.0f);
+      p.rng.state = 0;
+    }
+    stRec(pool.ray, slot, make_float4(p.o.x, p.o.y, p.o.z, p.d.x),
+          make_float4(p.d.y, p.d.z, bitsF((unsigned)p.rng.state),
+                      bitsF((unsigned)(p.rng.state >> 32))));
   }
 }
 
-// Stores a closest-hit candidate straight into the slot's hit record (three
-// 16-byte stores), so the trace loop keeps no hit fields in registers: each
-// closer hit overwrites the record, and a ray that hits nothing leaves the
-// miss marker (inst = -1) written when it was fetched.
-__device__ __forceinline__ void putHit(PoolSlot<TraceHit>& s, float t, int inst, int prim, float u,
+// Slot of ray i of the live list: the identity for the camera rays.
+template <bool CAM>
+__device__ __forceinline__ int liveSlot(int it, unsigned i) {
+  return CAM ? (int)i : c_pool.lists[it & 1][i];
+}
+
+// Stores a closest-hit candidate straight into the slot's hit record (one
+// 32-byte store), so the trace loop keeps no hit fields in registers: each
+// closer hit overwrites the record, and a ray whose tmax was never lowered
+// stores the miss marker when it ends.
+__device__ __forceinline__ void putHit(float4* hits, int slot, float t, int inst, int prim, float u,
                                        float v, float3 nq, bool front) {
-  static_assert(offsetof(TraceHit, nq) == 20 && offsetof(TraceHit, front) == 32 &&
-                    sizeof(PoolSlot<TraceHit>) == 48,
-                "TraceHit layout assumed by the vector stores");
-  float4* p = reinterpret_cast<float4*>(&s);
-  p[0] = make_float4(t, __int_as_float(inst), __int_as_float(prim), u);
-  p[1] = make_float4(v, nq.x, nq.y, nq.z);
-  p[2] = make_float4(__int_as_float(front ? 1 : 0), 0.0f, 0.0f, 0.0f);
+  stRec(hits, slot,
+        make_float4(t, __int_as_float(inst),
+                    bitsF((unsigned)prim | (front ? 0x80000000u : 0u)), u),
+        make_float4(v, nq.x, nq.y, nq.z));
+}
+__device__ __forceinline__ void putMiss(float4* hits, int slot) {
+  hits[2 * (size_t)slot] = make_float4(0.0f, __int_as_float(kMiss), 0.0f, 0.0f);
 }
 
 // Steps a lane may take in a row inside one round of the fetch loop, and
@@ -241,22 +216,21 @@ __device__ __forceinline__ void putHit(PoolSlot<TraceHit>& s, float t, int inst,
 // tests the 8 child boxes of the nearest remaining child node, or pops a
 // group. The visit order and tests are those of traverse<false> in the
 // 8-wide build: the same closest accepted hit.
-template <bool SERVE>
-__global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetch(int in) {
+template <bool SERVE, bool CAM>
+__global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetch(int it) {
   const WfPool& pool = c_pool;
-  const unsigned n = pool.counts[in];
+  const unsigned n = pool.counts[it].live;
   const unsigned full = 0xFFFFFFFFu;
   const unsigned ltMask = (1u << (threadIdx.x & 31)) - 1u;
   int job = 0;  // SERVE: the lane's job slot
   const float tmin = 0.0f;
-  unsigned long long rays = 0;
   int slot = -1;
   bool exhausted = false;  // warp-uniform
   float3 O = v3(0.0f), D = v3(0.0f);
   RayCtx ray;
   rayInit(ray, O, v3(1.0f), false);
   float tmax = 0.0f;
-  TraceHit hit;
+  TraceHit hit = {};
   bool found = false, inBlas = false;
   int curInst = -1, sp = 0;
   uint32_t gBase = 0, gHits = 0, gImask = 0, tBase = 0, tBits = 0;
@@ -266,17 +240,19 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetc
     if (!exhausted && (idle == full || __popc(idle) >= SDB_WF_FETCH_IDLE)) {
       const int leader = __ffs(idle) - 1;
       unsigned base = 0;
-      if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(&pool.counts[3], (unsigned)__popc(idle));
+      if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(&pool.counts[it].fetchRay, (unsigned)__popc(idle));
       base = __shfl_sync(full, base, leader);
       if (base + __popc(idle) >= n) exhausted = true;
       if (slot < 0) {
         unsigned i = base + __popc(idle & ltMask);
         if (i < n) {
-          slot = pool.lists[in][i];
+          slot = liveSlot<CAM>(it, i);
           if (SERVE) job = pool.jobs[slot];
           const SdLaunch& jl = SERVE ? c_wjobs[job] : c_wlp;
-          O = pool.paths[slot].v.o;
-          D = pool.paths[slot].v.d;
+          const Rec r = ldRec(pool.ray, slot);
+          O = v3(r.a.x, r.a.y, r.a.z);
+          D = v3(r.a.w, r.b.x, r.b.y);
+          if (CAM && D.x == 0.0f && D.y == 0.0f && D.z == 0.0f) slot = -1;  // tile padding
           rayInit(ray, O, D, false);
           tmax = 1e16f;
           found = false;
@@ -378,9 +354,8 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetc
       continue;
     }
     if (sp == 0) {  // ray done
-      if (!found) hit.inst = -1;
-      pool.hits[slot].v = hit;
-      rays++;
+      if (found) putHit(pool.hits, slot, hit.t, hit.inst, hit.prim, hit.u, hit.v, hit.nq, hit.front);
+      else putMiss(pool.hits, slot);
       slot = -1;
       continue;
     }
@@ -397,7 +372,6 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetc
       gImask = (e.y >> 8) & 0xFFu;
     }
   }
-  addRays<SERVE ? kWfServe : 0>(rays);
 }
 #else
 // Sink of the trace stage's walks (binTravStep, sd_trace.cuh): closer hits go
@@ -407,24 +381,29 @@ struct PoolSink {
   const WfPool& pool;
   int slot;
   __device__ __forceinline__ void world(float3& ro, float3& rd) const {
-    ro = pool.paths[slot].v.o;
-    rd = pool.paths[slot].v.d;
+    const Rec r = ldRec(pool.ray, slot);
+    ro = v3(r.a.x, r.a.y, r.a.z);
+    rd = v3(r.a.w, r.b.x, r.b.y);
   }
-  __device__ __forceinline__ float3 worldDir() const { return pool.paths[slot].v.d; }
+  __device__ __forceinline__ float3 worldDir() const {
+    const Rec r = ldRec(pool.ray, slot);
+    return v3(r.a.w, r.b.x, r.b.y);
+  }
   __device__ __forceinline__ void hit(float t, int inst, int prim, float u, float v, float3 nq,
                                       bool front) const {
-    putHit(pool.hits[slot], t, inst, prim, u, v, nq, front);
+    putHit(pool.hits, slot, t, inst, prim, u, v, nq, front);
   }
 };
 
-template <bool SERVE>
-__global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetch(int in) {
+constexpr float kRayMax = 1e16f;  // tmax of a radiance ray: any hit lowers it
+
+template <bool SERVE, bool CAM>
+__global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetch(int it) {
   const WfPool& pool = c_pool;
-  const unsigned n = pool.counts[in];
+  const unsigned n = pool.counts[it].live;
   const unsigned full = 0xFFFFFFFFu;
   const unsigned ltMask = (1u << (threadIdx.x & 31)) - 1u;
   int job = 0;  // SERVE: the lane's job slot
-  unsigned long long rays = 0;
   int slot = -1;
   bool exhausted = false;  // warp-uniform
   BinTrav t;
@@ -436,17 +415,20 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetc
     if (!exhausted && (idle == full || __popc(idle) >= SDB_WF_FETCH_IDLE)) {
       const int leader = __ffs(idle) - 1;
       unsigned base = 0;
-      if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(&pool.counts[3], (unsigned)__popc(idle));
+      if ((int)(threadIdx.x & 31) == leader)
+        base = atomicAdd(&pool.counts[it].fetchRay, (unsigned)__popc(idle));
       base = __shfl_sync(full, base, leader);
       if (base + __popc(idle) >= n) exhausted = true;
       if (slot < 0) {
         unsigned i = base + __popc(idle & ltMask);
         if (i < n) {
-          slot = pool.lists[in][i];
+          slot = liveSlot<CAM>(it, i);
           if (SERVE) job = pool.jobs[slot];
           const SdLaunch& jl = SERVE ? c_wjobs[job] : c_wlp;
-          binTravStart(t, jl, pool.paths[slot].v.o, pool.paths[slot].v.d, 1e16f);
-          pool.hits[slot].v.inst = -1;  // a miss until a hit is stored
+          const Rec r = ldRec(pool.ray, slot);
+          const float3 o = v3(r.a.x, r.a.y, r.a.z), d = v3(r.a.w, r.b.x, r.b.y);
+          binTravStart(t, jl, o, d, kRayMax);
+          if (CAM && d.x == 0.0f && d.y == 0.0f && d.z == 0.0f) slot = -1;  // tile padding
         }
       }
     }
@@ -469,51 +451,376 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetc
       if (k >= SDB_WF_INNER || __popc(__ballot_sync(full, go)) < SDB_WF_INNER_MIN) break;
     }
     if (slot >= 0 && r == kTravDone) {
-      rays++;  // its closest hit is already in the slot
+      if (t.tmax == kRayMax) putMiss(pool.hits, slot);
       slot = -1;
     }
   }
-  addRays<SERVE ? kWfServe : 0>(rays);
 }
 #endif
 
+// ---- shading ---------------------------------------------------------------------
+
+// Rays of a tile, shaded together by one block: sorted by what their hit
+// needs (kClass*), so a warp runs one material's code instead of stepping
+// through all of them with a few lanes each.
+constexpr int kTileMax = 8 * kRenderBlock;
+constexpr int kClasses = 8;       // miss, then 1 + MatKind, then tile padding
+constexpr int kClassNone = 7;
+constexpr int kWarps = kRenderBlock / 32;
+
+// Hides a value from the optimiser as a trip through memory does: the two
+// halves of a vertex round the same whether one kernel computes both or the
+// second runs later from stored state (no product of the first half fuses
+// into a sum of the second).
+__device__ __forceinline__ void opaque(float& x) { asm volatile("" : "+f"(x)); }
+__device__ __forceinline__ void opaque(int& x) { asm volatile("" : "+r"(x)); }
+__device__ __forceinline__ void opaque(float3& a) {
+  opaque(a.x);
+  opaque(a.y);
+  opaque(a.z);
+}
+
+__device__ __forceinline__ unsigned long long rngInc(const SdLaunch& lp) {
+  return ((unsigned long long)lp.seed << 1) | 1ull;  // Pcg::seeded's stream
+}
+
+// The finished path's sample; record passes also turn its trail of guided
+// vertices into training records.
 template <int GUIDE>
-__global__ void __launch_bounds__(kRenderBlock, SDB_WF_SHADE_BLOCKS) wfShadeA(int in, int out) {
-  const WfPool& pool = c_pool;
-  const unsigned n = pool.counts[in];
-  unsigned long long rays = 0;
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    int slot = pool.lists[in][i];
-    const SdLaunch& lp = slotLaunch<GUIDE>(slot);
-    Path p = pool.paths[slot].v;
-    TraceHit h = pool.hits[slot].v;
-    Vertex v;
-    if (shadeVertex<false>(lp, p, h.inst >= 0, h, rays, v)) {
-      pool.paths[slot].v = p;
-      pool.verts[slot].v = v;
-      pool.pending[slot] = 1;
-      if (v.nee) pool.shadowList[appendSlot(&pool.counts[2])] = slot;
-    } else {
-      finishPath<GUIDE>(p, slot);
-      pool.pending[slot] = 0;
-      refill<GUIDE>(slot, out);
-    }
+__device__ __forceinline__ void finishPath(float3 radiance, int sample, int slot) {
+  float3 L = sanitize3(radiance);
+  if (GUIDE & kGuideRecord) guideFlush(c_wlp, c_pool.trails[slot].v, L);
+  float4* sampleL = (GUIDE & kWfServe) ? c_wbatch.sampleL : c_wlp.sampleL;
+  sampleL[sample] = make_float4(L.x, L.y, L.z, 1.0f);
+}
+
+__device__ __forceinline__ void storeSum(const WfPool& pool, const Path& p, int slot) {
+  stRec(pool.sum, slot, make_float4(p.L.x, p.L.y, p.L.z, __int_as_float(p.slot)),
+        make_float4(p.beta.x, p.beta.y, p.beta.z, 0.0f));
+}
+__device__ __forceinline__ void storePath(const WfPool& pool, const Path& p, int slot) {
+  stRec(pool.ray, slot, make_float4(p.o.x, p.o.y, p.o.z, p.d.x),
+        make_float4(p.d.y, p.d.z, p.prevPdf,
+                    bitsF((p.specular ? 1u : 0u) | ((unsigned)p.medDepth << 1))));
+  storeSum(pool, p, slot);
+  stRec(pool.rest, slot, make_float4(p.prevX.x, p.prevX.y, p.prevX.z, 0.0f),
+        make_float4(bitsF((unsigned)p.rng.state), bitsF((unsigned)(p.rng.state >> 32)),
+                    bitsF((unsigned)p.med), bitsF((unsigned)(p.med >> 32))));
+}
+__device__ __forceinline__ unsigned long long join64(float lo, float hi) {
+  return (unsigned long long)bitsU(lo) | ((unsigned long long)bitsU(hi) << 32);
+}
+// The path in `slot` at `depth` (not a camera ray).
+__device__ __forceinline__ void loadPath(const WfPool& pool, const SdLaunch& lp, int slot, int depth,
+                                         Path& p) {
+  const Rec r = ldRec(pool.ray, slot), s = ldRec(pool.sum, slot), q = ldRec(pool.rest, slot);
+  p.o = v3(r.a.x, r.a.y, r.a.z);
+  p.d = v3(r.a.w, r.b.x, r.b.y);
+  p.prevPdf = r.b.z;
+  p.specular = (bitsU(r.b.w) & 1u) != 0;
+  p.medDepth = (int)(bitsU(r.b.w) >> 1);
+  p.L = v3(s.a.x, s.a.y, s.a.z);
+  p.slot = __float_as_int(s.a.w);
+  p.beta = v3(s.b.x, s.b.y, s.b.z);
+  p.prevX = v3(q.a.x, q.a.y, q.a.z);
+  p.rng.state = join64(q.b.x, q.b.y);
+  p.rng.inc = rngInc(lp);
+  p.med = join64(q.b.z, q.b.w);
+  p.depth = depth;
+  opaque(p.depth);
+}
+// The camera path with id `id` in `slot`.
+template <int GUIDE>
+__device__ __forceinline__ void loadCamera(const WfPool& pool, const SdLaunch& lp, int slot,
+                                           unsigned long long id, Path& p) {
+  const Rec r = ldRec(pool.ray, slot);
+  p.o = v3(r.a.x, r.a.y, r.a.z);
+  p.d = v3(r.a.w, r.b.x, r.b.y);
+  p.rng.state = join64(r.b.z, r.b.w);
+  p.rng.inc = rngInc(lp);
+  p.beta = v3(1.0f);
+  p.L = v3(0.0f);
+  p.prevX = p.o;
+  p.prevPdf = 0.0f;
+  p.specular = true;
+  p.med = 0ull;
+  p.medDepth = 0;
+  p.depth = 0;
+  if (GUIDE & kWfServe) {
+    p.slot = (int)id;
+  } else {
+    int px, py, s;
+    pathPixel(lp, id, px, py, s);
+    p.slot = sampleSlot(lp, px, py, s);
   }
-  addRays<GUIDE>(rays);
+  opaque(p.beta);
+  opaque(p.L);
+  opaque(p.prevPdf);
+  int specular = 1;
+  opaque(specular);
+  p.specular = specular != 0;
+  opaque(p.depth);
+}
+
+constexpr unsigned kShadowFinal = 1u;  // shadow ray flags: its path has ended
+constexpr unsigned kShadowLate = 2u;   // its vertex is finished by wfLate
+
+// One ray's shading. Returns what follows: bit 0 the path lives on, bit 1 it
+// queued a shadow ray, bit 2 its vertex waits for that ray.
+template <int GUIDE, bool CAM>
+__device__ __forceinline__ unsigned shadeRay(const WfPool& pool, int slot, unsigned long long id,
+                                             int depth) {
+  const SdLaunch& lp = slotLaunch<GUIDE>(slot);
+  Path p;
+  if (CAM) loadCamera<GUIDE>(pool, lp, slot, id, p);
+  else loadPath(pool, lp, slot, depth, p);
+  if (CAM && (GUIDE & kGuideRecord)) pool.trails[slot].v.n = 0;
+  const Rec hr = ldRec(pool.hits, slot);
+  TraceHit h;
+  h.t = hr.a.x;
+  h.inst = __float_as_int(hr.a.y);
+  h.prim = (int)(bitsU(hr.a.z) & 0x7FFFFFFFu);
+  h.front = (bitsU(hr.a.z) >> 31) != 0;
+  h.u = hr.a.w;
+  h.v = hr.b.x;
+  h.nq = v3(hr.b.y, hr.b.z, hr.b.w);
+  const bool hit = h.inst >= 0;
+  crossMedia(lp, p, hit, h.t);
+  Vertex v;
+  unsigned long long raysUnused = 0;
+  if (!shadeSurface(lp, p, hit, h, raysUnused, v)) {
+    finishPath<GUIDE>(p.L, p.slot, slot);
+    return 0;
+  }
+  const bool late = v.nee && ((GUIDE & kGuideRecord) || (lp.numFlames > 0 && lp.transparentShadows));
+  if (v.nee)
+    stRec(pool.shadowRays, slot, make_float4(v.so.x, v.so.y, v.so.z, v.wi.x),
+          make_float4(v.wi.y, v.wi.z, v.tmaxS, bitsF(late ? kShadowLate : 0u)));
+  if (late) {
+    storePath(pool, p, slot);
+    pool.verts[slot].v = v;
+    return 6;
+  }
+  int flags = (v.nee ? 1 : 0) | (v.delta ? 2 : 0) | (v.front ? 4 : 0);
+  opaque(flags);
+  v.nee = (flags & 1) != 0;
+  v.delta = (flags & 2) != 0;
+  v.front = (flags & 4) != 0;
+  opaque(v.matId);
+  opaque(v.x);
+  opaque(v.ns);
+  opaque(v.albedo);
+  opaque(v.etaExt);
+  opaque(v.etaRel);
+  opaque(v.wi);
+  opaque(v.Li);
+  opaque(v.pdf);
+  opaque(v.cosS);
+  opaque(p.beta);
+  opaque(p.L);
+  const SdMaterial mat = lp.materials[v.matId];
+  if (v.nee) {
+    const float3 c = neeTerm(lp, p, mat, v);
+    pool.shadowTerms[slot] = make_float4(c.x, c.y, c.z, 0.0f);
+  }
+  GuideTrail* trail = (GUIDE & kGuideRecord) ? &pool.trails[slot].v : nullptr;
+  if (sampleNext<GUIDE, kRound<GUIDE>>(lp, p, mat, v, trail)) {
+    storePath(pool, p, slot);
+    return v.nee ? 3 : 1;
+  }
+  if (v.nee) {  // the shadow ray adds the last term and finishes the sample
+    pool.sum[2 * (size_t)slot] = make_float4(p.L.x, p.L.y, p.L.z, __int_as_float(p.slot));
+    reinterpret_cast<unsigned*>(pool.shadowRays + 2 * (size_t)slot)[7] = kShadowFinal;
+    return 2;
+  }
+  finishPath<GUIDE>(p.L, p.slot, slot);
+  return 0;
+}
+
+// What the shading of a traced ray runs: 0 a miss, 1 + the kind of the hit
+// face's material, kClassNone for tile padding.
+template <int GUIDE>
+__device__ __forceinline__ int hitClass(const WfPool& pool, int slot) {
+  const float4 h = pool.hits[2 * (size_t)slot];
+  const int inst = __float_as_int(h.y);
+  if (inst < 0) return inst == kNoPath ? kClassNone : 0;
+  const SdLaunch& lp = slotLaunch<GUIDE>(slot);
+  const unsigned mats = lp.inst[inst].mats;
+  const unsigned m = (bitsU(h.z) >> 31) ? (mats & 0xFFFFu) : (mats >> 16);
+  return 1 + lp.materials[m].kind;
+}
+
+// Exclusive prefix sum of v over the calling warp; total gets the sum.
+__device__ __forceinline__ unsigned warpPrefix(unsigned v, unsigned& total) {
+  const int lane = threadIdx.x & 31;
+  unsigned x = v;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const unsigned y = __shfl_up_sync(0xFFFFFFFFu, x, off);
+    if (lane >= off) x += y;
+  }
+  total = __shfl_sync(0xFFFFFFFFu, x, 31);
+  return x - v;
+}
+
+// Shades the rays of the live list, a tile of up to kTileMax consecutive
+// list entries per block at a time: the tile is sorted by class in shared
+// memory and shaded in that order, and what lives on (and the shadow rays)
+// joins the next lists in the tile's own order, so the pixel order of the
+// camera rays is kept from bounce to bounce. Small lists take smaller tiles
+// so that every block has one.
+template <int GUIDE, bool CAM>
+__global__ void __launch_bounds__(kRenderBlock, SDB_WF_SHADE_BLOCKS) wfShade(
+    int it, int depth, unsigned long long base) {
+  __shared__ int sSlot[kTileMax];
+  __shared__ unsigned short sKey[kTileMax];    // class << 8 | rank; then the sorted order
+  __shared__ unsigned char sFlag[kTileMax];
+  __shared__ unsigned short sOrder[kTileMax];
+  constexpr int kGroups = kTileMax / 32;       // warps' worth of entries in a tile
+  __shared__ unsigned short sCount[kClasses * kGroups];
+  __shared__ unsigned sList[3][kGroups];
+  __shared__ unsigned sBase[3];
+  __shared__ unsigned sPart[kWarps];
+  const WfPool& pool = c_pool;
+  WfCounts& cnt = pool.counts[it];
+  const unsigned full = 0xFFFFFFFFu;
+  const unsigned n = cnt.live;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned ltMask = (1u << lane) - 1u;
+  const unsigned per = (n + gridDim.x * kRenderBlock - 1) / (gridDim.x * kRenderBlock);
+  // Record passes keep the records of the paths that end first: small tiles
+  // there, so those are not the misses of large ones.
+  const unsigned most = (GUIDE & kGuideRecord) ? 1u : (unsigned)(kTileMax / kRenderBlock);
+  const int K = (int)min(max(per, 1u), most);
+  const unsigned T = (unsigned)K * kRenderBlock;
+  for (unsigned t0 = blockIdx.x * T; t0 < n; t0 += gridDim.x * T) {
+    // Classes, and each entry's rank among its warp's entries of the class.
+    for (int k = tid; k < kClasses * kGroups; k += kRenderBlock) sCount[k] = 0;
+    __syncthreads();
+    for (int k = 0; k < K; k++) {
+      const int e = k * kRenderBlock + tid;
+      const unsigned i = t0 + e;
+      int slot = -1, cls = kClassNone;
+      if (i < n) {
+        slot = liveSlot<CAM>(it, i);
+        cls = hitClass<GUIDE>(pool, slot);
+      }
+      const unsigned same = __match_any_sync(full, cls);
+      const int rank = __popc(same & ltMask);
+      if (rank == 0) sCount[cls * kGroups + (e >> 5)] = (unsigned short)__popc(same);
+      sSlot[e] = slot;
+      sKey[e] = (unsigned short)(cls << 8 | rank);
+      sFlag[e] = 0;
+    }
+    __syncthreads();
+    // Prefix over the counts, class by class (two entries per thread).
+    static_assert(kClasses * kGroups == 2 * kRenderBlock, "two counts per thread");
+    {
+      const unsigned c0 = sCount[2 * tid], c1 = sCount[2 * tid + 1];
+      unsigned total;
+      const unsigned ex = warpPrefix(c0 + c1, total);
+      if (lane == 0) sPart[warp] = total;
+      __syncthreads();
+      unsigned before = 0;
+      for (int w = 0; w < warp; w++) before += sPart[w];
+      sCount[2 * tid] = (unsigned short)(before + ex);
+      sCount[2 * tid + 1] = (unsigned short)(before + ex + c0);
+    }
+    __syncthreads();
+    const int shaded = sCount[kClassNone * kGroups];  // entries that hold a path
+    for (int k = 0; k < K; k++) {
+      const int e = k * kRenderBlock + tid;
+      const unsigned key = sKey[e];
+      sOrder[sCount[(key >> 8) * kGroups + (e >> 5)] + (key & 0xFFu)] = (unsigned short)e;
+    }
+    __syncthreads();
+    for (int j = tid; j < shaded; j += kRenderBlock) {
+      const int e = sOrder[j];
+      sFlag[e] = (unsigned char)shadeRay<GUIDE, CAM>(pool, sSlot[e], base + t0 + e, depth);
+    }
+    __syncthreads();
+    // The tile's contributions to the next lists, in its own order.
+    for (int k = 0; k < K; k++) {
+      const int e = k * kRenderBlock + tid;
+      const unsigned f = sFlag[e];
+      const unsigned live = __ballot_sync(full, f & 1u), shadow = __ballot_sync(full, f & 2u),
+                     late = __ballot_sync(full, f & 4u);
+      if (lane == 0) {
+        sList[0][e >> 5] = __popc(live);
+        sList[1][e >> 5] = __popc(shadow);
+        sList[2][e >> 5] = __popc(late);
+      }
+    }
+    __syncthreads();
+    if (warp < 3) {
+      unsigned total;
+      const bool in = lane < K * kWarps;
+      const unsigned ex = warpPrefix(in ? sList[warp][lane] : 0u, total);
+      if (in) sList[warp][lane] = ex;
+      if (lane == 0 && total) {
+        unsigned* c = warp == 0 ? &pool.counts[it + 1].live : (warp == 1 ? &cnt.shadow : &cnt.late);
+        sBase[warp] = atomicAdd(c, total);
+      }
+      if (warp == 1 && lane == 0) {
+        unsigned long long* rays = (GUIDE & kWfServe) ? c_wbatch.rayCounter : c_wlp.rayCounter;
+        atomicAdd(rays, (unsigned long long)shaded + total);
+      }
+    } else if (lane == 0) {
+      atomicAdd(&cnt.traced, (unsigned)shaded);
+    }
+    __syncthreads();
+    for (int k = 0; k < K; k++) {
+      const int e = k * kRenderBlock + tid;
+      const unsigned f = sFlag[e];
+      const unsigned live = __ballot_sync(full, f & 1u), shadow = __ballot_sync(full, f & 2u),
+                     late = __ballot_sync(full, f & 4u);
+      const int slot = sSlot[e];
+      if (f & 1u) pool.lists[(it + 1) & 1][sBase[0] + sList[0][e >> 5] + __popc(live & ltMask)] = slot;
+      if (f & 2u) pool.shadowList[sBase[1] + sList[1][e >> 5] + __popc(shadow & ltMask)] = slot;
+      if (f & 4u) pool.lateList[sBase[2] + sList[2][e >> 5] + __popc(late & ltMask)] = slot;
+    }
+    __syncthreads();
+  }
+}
+
+// ---- shadow rays --------------------------------------------------------------------
+
+// A shadow ray's result: the transmittance to a late vertex, or its NEE term
+// added to the path's radiance, which for an ended path is its sample.
+template <int GUIDE>
+__device__ __forceinline__ void finishShadow(const WfPool& pool, int slot, unsigned flags, float3 tr,
+                                             int depth) {
+  if (flags & kShadowLate) {
+    pool.shadowTerms[slot] = make_float4(tr.x, tr.y, tr.z, 0.0f);
+    return;
+  }
+  const bool lit = hmax(tr) > 0.0f;
+  if (!lit && !(flags & kShadowFinal)) return;
+  float4 s = pool.sum[2 * (size_t)slot];
+  float3 L = v3(s.x, s.y, s.z);
+  if (lit) {
+    const float4 c = pool.shadowTerms[slot];
+    float3 z = v3(__fmul_rn(c.x, tr.x), __fmul_rn(c.y, tr.y), __fmul_rn(c.z, tr.z));
+    z = neeRadiance(z, v3(1.0f), depth >= 1, slotLaunch<GUIDE>(slot).clampVal);
+    L = v3(__fadd_rn(L.x, z.x), __fadd_rn(L.y, z.y), __fadd_rn(L.z, z.z));
+  }
+  if (flags & kShadowFinal) finishPath<GUIDE & kWfServe>(L, __float_as_int(s.w), slot);
+  else pool.sum[2 * (size_t)slot] = make_float4(L.x, L.y, L.z, s.w);
 }
 
 // Shadow rays, one per thread to the end of its walk (grid-stride over the
 // shadow list).
 template <int GUIDE>
-__global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfShadow() {
+__global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfShadow(int it, int depth) {
   const WfPool& pool = c_pool;
-  const unsigned n = pool.counts[2];
+  const unsigned n = pool.counts[it].shadow;
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     int slot = pool.shadowList[i];
     const SdLaunch& lp = slotLaunch<GUIDE>(slot);
-    const Vertex& v = pool.verts[slot].v;
-    float3 tr = shadowTransmittance<false>(lp, v.so, v.wi, v.tmaxS, nullptr);
-    pool.trs[slot] = make_float4(tr.x, tr.y, tr.z, 0.0f);
+    const Rec r = ldRec(pool.shadowRays, slot);
+    const float3 so = v3(r.a.x, r.a.y, r.a.z), wi = v3(r.a.w, r.b.x, r.b.y);
+    const float3 tr = shadowTransmittance<false>(lp, so, wi, r.b.z, nullptr);
+    finishShadow<GUIDE>(pool, slot, bitsU(r.b.w), tr, depth);
   }
 }
 
@@ -524,23 +831,27 @@ struct ShadowSink {
   const WfPool& pool;
   int slot;
   __device__ __forceinline__ void world(float3& ro, float3& rd) const {
-    ro = pool.verts[slot].v.so;
-    rd = pool.verts[slot].v.wi;
+    const Rec r = ldRec(pool.shadowRays, slot);
+    ro = v3(r.a.x, r.a.y, r.a.z);
+    rd = v3(r.a.w, r.b.x, r.b.y);
   }
-  __device__ __forceinline__ float3 worldDir() const { return pool.verts[slot].v.wi; }
+  __device__ __forceinline__ float3 worldDir() const {
+    const Rec r = ldRec(pool.shadowRays, slot);
+    return v3(r.a.w, r.b.x, r.b.y);
+  }
   __device__ __forceinline__ void hit(float, int, int, float, float, float3, bool) const {}
 };
 
-// Shadow rays with the trace stage's dynamic fetch (counter counts[4]) and
+// Shadow rays with the trace stage's dynamic fetch and
 // node-descent runs: the walk and transmittance of shadowTransmittance, many
 // rays interleaved per warp. Faster than wfShadow where walks are long and
 // uneven (config 1, 1024 instances: 29.3 -> 24.5 ms per frame), slower on
 // small scenes (config 0: 2,730 -> 2,672 Mrays/s; config 2: 113.7 -> 122.2
 // ms), so renders choose by instance count (kShadowFetchInstances).
 template <int GUIDE>
-__global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfShadowFetch() {
+__global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfShadowFetch(int it, int depth) {
   const WfPool& pool = c_pool;
-  const unsigned n = pool.counts[2];
+  const unsigned n = pool.counts[it].shadow;
   const unsigned full = 0xFFFFFFFFu;
   const unsigned ltMask = (1u << (threadIdx.x & 31)) - 1u;
   int slot = -1;
@@ -554,15 +865,17 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfShadowFet
     if (!exhausted && (idle == full || __popc(idle) >= SDB_WF_FETCH_IDLE)) {
       const int leader = __ffs(idle) - 1;
       unsigned base = 0;
-      if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(&pool.counts[4], (unsigned)__popc(idle));
+      if ((int)(threadIdx.x & 31) == leader)
+        base = atomicAdd(&pool.counts[it].fetchShadow, (unsigned)__popc(idle));
       base = __shfl_sync(full, base, leader);
       if (base + __popc(idle) >= n) exhausted = true;
       if (slot < 0) {
         unsigned i = base + __popc(idle & ltMask);
         if (i < n) {
           slot = pool.shadowList[i];
-          const Vertex& v = pool.verts[slot].v;
-          binTravStart(t, slotLaunch<GUIDE>(slot), v.so, v.wi, v.tmaxS);
+          const Rec r = ldRec(pool.shadowRays, slot);
+          binTravStart(t, slotLaunch<GUIDE>(slot), v3(r.a.x, r.a.y, r.a.z),
+                       v3(r.a.w, r.b.x, r.b.y), r.b.z);
           trProd = 1.0f;
           tau = v3(0.0f);
         }
@@ -588,7 +901,8 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfShadowFet
         tr = v3(trProd);
         if (hmax(tau) > 0.0f) tr = tr * vexp(-tau);
       }
-      pool.trs[slot] = make_float4(tr.x, tr.y, tr.z, 0.0f);
+      const unsigned flags = reinterpret_cast<const unsigned*>(pool.shadowRays + 2 * (size_t)slot)[7];
+      finishShadow<GUIDE>(pool, slot, flags, tr, depth);
       slot = -1;
     }
   }
@@ -596,37 +910,45 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfShadowFet
 #else
 // The 8-wide build traces shadow rays one per thread.
 template <int GUIDE>
-__global__ void wfShadowFetch() {}
+__global__ void wfShadowFetch(int, int) {}
 #endif
 
-// GUIDE & kGuideSample: the BSDF sample by MIS with the learned guide
-// (sd_guide.cuh; the mixture table is in the launch block). GUIDE &
-// kGuideRecord: the guided vertex joins the slot's trail.
+// Late vertices (their shadow ray's transmittance is in shadowTerms): the
+// NEE contribution, the BSDF sample, roulette. GUIDE & kGuideRecord: the
+// guided vertex joins the slot's trail.
 template <int GUIDE>
-__global__ void __launch_bounds__(kRenderBlock, SDB_WF_SHADEB_BLOCKS) wfShadeB(int in, int out) {
+__global__ void __launch_bounds__(kRenderBlock, SDB_WF_SHADE_BLOCKS) wfLate(int it, int depth) {
   const WfPool& pool = c_pool;
-  const unsigned n = pool.counts[in];
+  const unsigned n = pool.counts[it].late;
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    int slot = pool.lists[in][i];
-    if (!pool.pending[slot]) continue;
+    const int slot = pool.lateList[i];
     const SdLaunch& lp = slotLaunch<GUIDE>(slot);
-    Path p = pool.paths[slot].v;
+    Path p;
+    loadPath(pool, lp, slot, depth, p);
     const Vertex v = pool.verts[slot].v;
-    float3 tr = v3(0.0f);
-    if (v.nee) {
-      float4 t4 = pool.trs[slot];
-      tr = v3(t4.x, t4.y, t4.z);
-    }
+    const float4 tr = pool.shadowTerms[slot];
     GuideTrail* trail = (GUIDE & kGuideRecord) ? &pool.trails[slot].v : nullptr;
-    if (finishVertex<GUIDE>(lp, p, v, tr, trail)) {
-      pool.paths[slot].v = p;
-      pool.lists[out][appendSlot(&pool.counts[out])] = slot;
+    if (finishVertex<GUIDE, kRound<GUIDE>>(lp, p, v, v3(tr.x, tr.y, tr.z), trail)) {
+      storePath(pool, p, slot);
+      pool.lists[(it + 1) & 1][appendSlot(&pool.counts[it + 1].live)] = slot;
     } else {
-      finishPath<GUIDE>(p, slot);
-      refill<GUIDE>(slot, out);
+      finishPath<GUIDE>(p.L, p.slot, slot);
     }
   }
 }
+
+// Between two groups of iterations: the last list's length moves to the
+// front (kWfGroup is even, so the list keeps its place), the rest clears.
+__global__ void wfNextGroup() {
+  WfCounts* c = c_pool.counts;
+  const unsigned live = c[kWfGroup].live;
+  __syncwarp();
+  for (int k = threadIdx.x; k < (int)((kWfGroup + 1) * sizeof(WfCounts) / 4); k += 32)
+    reinterpret_cast<unsigned*>(c)[k] = 0;
+  __syncwarp();
+  if (threadIdx.x == 0) c[0].live = live;
+}
+static_assert(kWfGroup % 2 == 0, "lists ping-pong back to their place");
 
 // ---- host ---------------------------------------------------------------------
 
@@ -639,37 +961,58 @@ static int gridFor(K kernel) {
   return sms * (perSm < 1 ? 1 : perSm);
 }
 
-void WfBuffers::ensure(int slots) {
-  if (slots <= cap) return;
+bool wfHasLate(const SdLaunch& lp, int guide) {
+  return (guide & kGuideRecord) || (lp.numFlames > 0 && lp.transparentShadows);
+}
+
+void WfBuffers::ensure(int slots, bool withLate) {
+  if (slots <= cap && (late || !withLate)) return;
+  withLate = withLate || late;
+  slots = std::max(slots, cap);
   // At most half of the device memory that is free (counting the pool about
   // to be replaced), so films, scenes and other work keep room; at least
   // 1 M slots.
   size_t freeB = 0, totB = 0;
   cudaCheck(cudaMemGetInfo(&freeB, &totB), "cudaMemGetInfo");
-  const size_t budget = (freeB + (size_t)cap * wfSlotBytes()) / 2;
-  const size_t fit = std::max<size_t>(budget / wfSlotBytes(), (size_t)1 << 20);
+  const size_t budget = (freeB + (size_t)cap * wfSlotBytes(late)) / 2;
+  const size_t fit = std::max<size_t>(budget / wfSlotBytes(withLate), (size_t)1 << 20);
   slots = (int)std::min<size_t>((size_t)slots, fit);
-  if (slots <= cap) return;
+  if (slots <= cap && late == withLate) return;
   const size_t n = (size_t)slots;
-  const size_t sizes[9] = {n * sizeof(PoolSlot<Path>), n * sizeof(PoolSlot<Vertex>),
-                           n * sizeof(PoolSlot<TraceHit>), n * sizeof(float4), n,
-                           n * sizeof(int), n * sizeof(int), n * sizeof(int), n};
-  size_t offs[9], total = 0;
-  for (int k = 0; k < 9; k++) {
+  const size_t sizes[12] = {n * 32, n * 32, n * 32, n * 32, n * 32, n * 16,
+                            n * sizeof(int), n * sizeof(int), n * sizeof(int), n * sizeof(int), n,
+                            withLate ? n * sizeof(PoolSlot<Vertex>) : 0};
+  size_t offs[12], total = 0;
+  for (int k = 0; k < 12; k++) {
     offs[k] = total;
     total += (sizes[k] + 255) & ~(size_t)255;
   }
+  cap = 0;
+  late = false;
   slab.release();
   slab.alloc(total);
-  void** parts[9] = {&paths, &verts, &hits, &trs, &pending, &list0, &list1, &shadow, &jobs};
-  for (int k = 0; k < 9; k++) *parts[k] = (char*)slab.ptr + offs[k];
-  if (!counts.ptr) counts.alloc(8 * sizeof(unsigned));
+  char* base = (char*)slab.ptr;
+  pool.ray = (float4*)(base + offs[0]);
+  pool.sum = (float4*)(base + offs[1]);
+  pool.rest = (float4*)(base + offs[2]);
+  pool.hits = (float4*)(base + offs[3]);
+  pool.shadowRays = (float4*)(base + offs[4]);
+  pool.shadowTerms = (float4*)(base + offs[5]);
+  pool.lists[0] = (int*)(base + offs[6]);
+  pool.lists[1] = (int*)(base + offs[7]);
+  pool.shadowList = (int*)(base + offs[8]);
+  pool.lateList = (int*)(base + offs[9]);
+  pool.jobs = (unsigned char*)(base + offs[10]);
+  pool.verts = withLate ? (PoolSlot<Vertex>*)(base + offs[11]) : nullptr;
+  if (!counts.ptr) counts.alloc((kWfGroup + 1) * sizeof(WfCounts));
+  pool.counts = (WfCounts*)counts.ptr;
   if (!hostCount) hostCount = pinnedWords();
   cap = slots;
-  gridTrace = gridFor(wfTraceFetch<false>);
-  gridShadeA = gridFor(wfShadeA<0>);
+  late = withLate;
+  gridTrace = gridFor(wfTraceFetch<false, false>);
+  gridShade = gridFor(wfShade<0, false>);
   gridShadow = gridFor(wfShadow<0>);
-  gridShadeB = gridFor(wfShadeB<0>);
+  gridLate = gridFor(wfLate<0>);
   gridStart = gridFor(wfStart<0>);
 }
 
@@ -719,30 +1062,51 @@ void wfReleaseIdle() {
   cudaSetDevice(cur);
 }
 
-size_t wfSlotBytes() {
-  return sizeof(PoolSlot<Path>) + sizeof(PoolSlot<Vertex>) + sizeof(PoolSlot<TraceHit>) +
-         sizeof(float4) + 2 + 3 * sizeof(int);
+size_t wfSlotBytes(bool withLate) {
+  return 6 * 32 - 16 + 4 * sizeof(int) + 1 + (withLate ? sizeof(PoolSlot<Vertex>) : 0);
 }
 
-// Renders the launch block's paths (lp.numPaths ids, counters already
-// cleared) into lp.sampleL through the stages. Returns the kernels launched.
+// What the launches of a render or batch need.
+struct WfPlan {
+  int mode;           // guide bits, or kWfServe
+  bool shadowFetch;   // the shadow-ray kernel (kShadowFetchInstances)
+  bool lights;        // any NEE strategy: shadow rays can exist
+  bool late;          // late vertices can exist
+  int maxDepth;
+};
+
 // One iteration's stage kernels for mode GUIDE (guide bits, or kWfServe).
-// With `timed`, events ev[1..5] bracket the four stage launches.
-template <int GUIDE>
-static void wfIteration(const WfBuffers& b, cudaStream_t st, int cur, int nxt, bool timed,
-                        bool shadowFetch) {
+// With `timed`, events ev[1..5] bracket the stage launches.
+template <int GUIDE, bool CAM>
+static int wfIteration(const WfBuffers& b, cudaStream_t st, int it, int depth,
+                       unsigned long long base, const WfPlan& plan, bool timed) {
+  int launches = 2;
   if (timed) cudaEventRecord(b.ev[1], st);
-  wfTraceFetch<(GUIDE & kWfServe) != 0><<<b.gridTrace, kRenderBlock, 0, st>>>(cur);
+  wfTraceFetch<(GUIDE & kWfServe) != 0, CAM><<<b.gridTrace, kRenderBlock, 0, st>>>(it);
   if (timed) cudaEventRecord(b.ev[2], st);
-  wfShadeA<GUIDE><<<b.gridShadeA, kRenderBlock, 0, st>>>(cur, nxt);
+  wfShade<GUIDE, CAM><<<b.gridShade, kRenderBlock, 0, st>>>(it, depth, base);
   if (timed) cudaEventRecord(b.ev[3], st);
-  if (shadowFetch && !SDB_WIDE_BVH)
-    wfShadowFetch<GUIDE><<<b.gridShadow, kRenderBlock, 0, st>>>();
-  else
-    wfShadow<GUIDE><<<b.gridShadow, kRenderBlock, 0, st>>>();
+  if (plan.lights) {
+    if (plan.shadowFetch && !SDB_WIDE_BVH)
+      wfShadowFetch<GUIDE><<<b.gridShadow, kRenderBlock, 0, st>>>(it, depth);
+    else
+      wfShadow<GUIDE><<<b.gridShadow, kRenderBlock, 0, st>>>(it, depth);
+    launches++;
+  }
   if (timed) cudaEventRecord(b.ev[4], st);
-  wfShadeB<GUIDE><<<b.gridShadeB, kRenderBlock, 0, st>>>(cur, nxt);
+  if (plan.late) {
+    wfLate<GUIDE><<<b.gridLate, kRenderBlock, 0, st>>>(it, depth);
+    launches++;
+  }
   if (timed) cudaEventRecord(b.ev[5], st);
+  return launches;
+}
+
+template <int GUIDE>
+static int wfIterationAny(const WfBuffers& b, cudaStream_t st, int it, int depth,
+                          unsigned long long base, const WfPlan& plan, bool timed) {
+  return depth == 0 ? wfIteration<GUIDE, true>(b, st, it, depth, base, plan, timed)
+                    : wfIteration<GUIDE, false>(b, st, it, depth, base, plan, timed);
 }
 
 static double evMs(cudaEvent_t a, cudaEvent_t b) {
@@ -751,87 +1115,80 @@ static double evMs(cudaEvent_t a, cudaEvent_t b) {
   return ms;
 }
 
-// Fills the pool with the first paths of ids [0, numPaths) and runs stage
-// iterations until no path is live (the launch block or batch is already in
-// constant memory). Returns the kernels launched.
-static int runPool(WfBuffers& b, cudaStream_t st, unsigned long long numPaths, int mode,
-                   bool shadowFetch, bool directStart, WfStageTimes* times = nullptr) {
+// Renders path ids [0, numPaths), a pool of them at a time, each through
+// stage iterations until no path is live (the launch block or batch is
+// already in constant memory). Paths of a pool share their depth, so
+// plan.maxDepth iterations end them all; in groups of kWfGroup, with a look
+// at the live count between groups. Returns the kernels launched.
+static int runPool(WfBuffers& b, cudaStream_t st, unsigned long long numPaths, const WfPlan& plan,
+                   WfStageTimes* times = nullptr) {
   const bool timed = times != nullptr;
   if (timed && !b.ev[0])
     for (cudaEvent_t& e : b.ev) cudaCheck(cudaEventCreate(&e), "stage timing events");
-  WfPool pool;
-  pool.paths = (PoolSlot<Path>*)b.paths;
-  pool.verts = (PoolSlot<Vertex>*)b.verts;
-  pool.hits = (PoolSlot<TraceHit>*)b.hits;
-  pool.trs = (float4*)b.trs;
-  pool.pending = (unsigned char*)b.pending;
-  pool.lists[0] = (int*)b.list0;
-  pool.lists[1] = (int*)b.list1;
-  pool.shadowList = (int*)b.shadow;
-  pool.counts = (unsigned*)b.counts.ptr;
+  WfPool pool = b.pool;
   pool.trails = (PoolSlot<GuideTrail>*)b.trails.ptr;
-  pool.jobs = (unsigned char*)b.jobs;
-  pool.cap = (int)std::min<unsigned long long>((unsigned long long)b.cap, numPaths);
-  pool.refillOpen = (unsigned long long)pool.cap < numPaths ? 1 : 0;
   cudaCheck(cudaMemcpyToSymbolAsync(c_pool, &pool, sizeof pool, 0, cudaMemcpyHostToDevice, st),
             "wavefront pool");
-  cudaCheck(cudaMemsetAsync(b.counts.ptr, 0, b.counts.bytes, st), "wavefront counts");
   int launches = 0;
-  if (timed) cudaEventRecord(b.ev[0], st);
-  const unsigned direct = (unsigned)pool.cap;
-  if (mode & kWfServe)
-    wfStart<kWfServe><<<b.gridStart, kRenderBlock, 0, st>>>();
-  else if (directStart && (mode & kGuideRecord))
-    wfStartDirect<kGuideRecord><<<b.gridStart, kRenderBlock, 0, st>>>(direct);
-  else if (directStart)
-    wfStartDirect<0><<<b.gridStart, kRenderBlock, 0, st>>>(direct);
-  else if (mode & kGuideRecord)
-    wfStart<kGuideRecord><<<b.gridStart, kRenderBlock, 0, st>>>();
-  else
-    wfStart<0><<<b.gridStart, kRenderBlock, 0, st>>>();
-  cudaCheck(cudaGetLastError(), "wfStart");
-  launches++;
-  if (timed) {
-    cudaEventRecord(b.ev[1], st);
-    cudaCheck(cudaEventSynchronize(b.ev[1]), "wfStart");
-    times->startMs += evMs(b.ev[0], b.ev[1]);
-    times->launches++;
-  }
-  unsigned* counts = (unsigned*)b.counts.ptr;
-  int cur = 0;
-  for (int iter = 0;; iter++) {
-    int nxt = 1 - cur;
-    cudaCheck(cudaMemsetAsync(counts + nxt, 0, sizeof(unsigned), st), "wavefront counts");
-    cudaCheck(cudaMemsetAsync(counts + 2, 0, 3 * sizeof(unsigned), st), "wavefront counts");
-    switch (mode) {
-      case 0: wfIteration<0>(b, st, cur, nxt, timed, shadowFetch); break;
-      case kGuideSample: wfIteration<kGuideSample>(b, st, cur, nxt, timed, shadowFetch); break;
-      case kGuideRecord: wfIteration<kGuideRecord>(b, st, cur, nxt, timed, shadowFetch); break;
-      case kGuideSample | kGuideRecord:
-        wfIteration<kGuideSample | kGuideRecord>(b, st, cur, nxt, timed, shadowFetch);
-        break;
-      default: wfIteration<kWfServe>(b, st, cur, nxt, timed, shadowFetch); break;
-    }
-    cudaCheck(cudaGetLastError(), "wavefront stage");
-    launches += 4;
-    cur = nxt;
-    // All four counters: [cur] is now the next iteration's live list, [1 - cur]
-    // the list this iteration traced, [2] its shadow rays.
-    cudaCheck(cudaMemcpyAsync(b.hostCount, counts, 4 * sizeof(unsigned), cudaMemcpyDeviceToHost, st),
-              "wavefront count");
-    cudaCheck(cudaStreamSynchronize(st), "wavefront iteration");
+  for (unsigned long long base = 0; base < numPaths; base += (unsigned long long)b.cap) {
+    const unsigned n = (unsigned)std::min<unsigned long long>((unsigned long long)b.cap,
+                                                              numPaths - base);
+    cudaCheck(cudaMemsetAsync(b.counts.ptr, 0, b.counts.bytes, st), "wavefront counts");
+    if (timed) cudaEventRecord(b.ev[0], st);
+    if (plan.mode & kWfServe) wfStart<kWfServe><<<b.gridStart, kRenderBlock, 0, st>>>(base, n);
+    else wfStart<0><<<b.gridStart, kRenderBlock, 0, st>>>(base, n);
+    cudaCheck(cudaGetLastError(), "wfStart");
+    launches++;
     if (timed) {
-      times->traceMs += evMs(b.ev[1], b.ev[2]);
-      times->shadeAMs += evMs(b.ev[2], b.ev[3]);
-      times->shadowMs += evMs(b.ev[3], b.ev[4]);
-      times->shadeBMs += evMs(b.ev[4], b.ev[5]);
-      times->iterations++;
-      times->launches += 4;
-      times->radianceRays += b.hostCount[1 - cur];
-      times->shadowRays += b.hostCount[2];
+      cudaEventRecord(b.ev[1], st);
+      cudaCheck(cudaEventSynchronize(b.ev[1]), "wfStart");
+      times->startMs += evMs(b.ev[0], b.ev[1]);
+      times->launches++;
     }
-    if (b.hostCount[cur] == 0) break;
-    if (iter > (1 << 24)) throw std::runtime_error("wavefront: no progress");
+    for (int depth = 0;; depth++) {
+      const int it = depth % kWfGroup;
+      if (depth > 0 && it == 0) {  // the next group of iterations
+        unsigned* live = &((WfCounts*)b.counts.ptr)[kWfGroup].live;
+        cudaCheck(cudaMemcpyAsync(b.hostCount, live, sizeof(unsigned), cudaMemcpyDeviceToHost, st),
+                  "wavefront count");
+        cudaCheck(cudaStreamSynchronize(st), "wavefront group");
+        if (b.hostCount[0] == 0) break;
+        wfNextGroup<<<1, 32, 0, st>>>();
+        launches++;
+      }
+      int k;
+      switch (plan.mode) {
+        case 0: k = wfIterationAny<0>(b, st, it, depth, base, plan, timed); break;
+        case kGuideSample:
+          k = wfIterationAny<kGuideSample>(b, st, it, depth, base, plan, timed);
+          break;
+        case kGuideRecord:
+          k = wfIterationAny<kGuideRecord>(b, st, it, depth, base, plan, timed);
+          break;
+        case kGuideSample | kGuideRecord:
+          k = wfIterationAny<kGuideSample | kGuideRecord>(b, st, it, depth, base, plan, timed);
+          break;
+        default: k = wfIterationAny<kWfServe>(b, st, it, depth, base, plan, timed); break;
+      }
+      cudaCheck(cudaGetLastError(), "wavefront stage");
+      launches += k;
+      if (timed) {
+        static_assert(offsetof(WfCounts, traced) == 3 * sizeof(unsigned), "counter order");
+        cudaCheck(cudaMemcpyAsync(b.hostCount, (WfCounts*)b.counts.ptr + it, 4 * sizeof(unsigned),
+                                  cudaMemcpyDeviceToHost, st),
+                  "wavefront count");
+        cudaCheck(cudaStreamSynchronize(st), "wavefront iteration");
+        times->traceMs += evMs(b.ev[1], b.ev[2]);
+        times->shadeAMs += evMs(b.ev[2], b.ev[3]);
+        times->shadowMs += evMs(b.ev[3], b.ev[4]);
+        times->shadeBMs += evMs(b.ev[4], b.ev[5]);
+        times->iterations++;
+        times->launches += k;
+        times->radianceRays += b.hostCount[3];
+        times->shadowRays += b.hostCount[1];
+      }
+      if (depth + 1 >= plan.maxDepth) break;
+    }
   }
   return launches;
 }
@@ -842,9 +1199,10 @@ int wfRender(const SdLaunch& lp, WfBuffers& b, cudaStream_t st, int guide, WfSta
   if (guide & kGuideRecord) b.ensureTrails();
   cudaCheck(cudaMemcpyToSymbolAsync(c_wlp, &lp, sizeof lp, 0, cudaMemcpyHostToDevice, st),
             "wavefront launch block");
-  const bool exactTiles = lp.shardCount <= 1 && lp.npixPad == lp.width * lp.height;
-  return runPool(b, st, lp.numPaths, guide, lp.numInstances >= kShadowFetchInstances, exactTiles,
-                 times);
+  const WfPlan plan = {guide, lp.numInstances >= kShadowFetchInstances,
+                       lp.numLights > 0 || lp.bgKind == BG_ENVMAP, wfHasLate(lp, guide),
+                       lp.maxDepth};
+  return runPool(b, st, lp.numPaths, plan, times);
 }
 
 cudaError_t wfSetJobs(const SdLaunch* table, cudaStream_t st) {
@@ -852,10 +1210,18 @@ cudaError_t wfSetJobs(const SdLaunch* table, cudaStream_t st) {
                                  cudaMemcpyHostToDevice, st);
 }
 
-int wfRenderBatch(const ServeBatch& batch, WfBuffers& b, cudaStream_t st, int maxInstances) {
+int wfRenderBatch(const ServeBatch& batch, WfBuffers& b, cudaStream_t st, const SdLaunch* jobs) {
   cudaCheck(cudaMemcpyToSymbolAsync(c_wbatch, &batch, sizeof batch, 0, cudaMemcpyHostToDevice, st),
             "wavefront batch");
-  return runPool(b, st, batch.numPaths, kWfServe, maxInstances >= kShadowFetchInstances, false);
+  WfPlan plan = {kWfServe, false, false, false, 0};
+  for (int k = 0; k < kMaxServeJobs; k++) {  // unused slots are zero
+    const SdLaunch& lp = jobs[k];
+    plan.shadowFetch = plan.shadowFetch || lp.numInstances >= kShadowFetchInstances;
+    plan.lights = plan.lights || lp.numLights > 0 || (lp.width > 0 && lp.bgKind == BG_ENVMAP);
+    plan.late = plan.late || wfHasLate(lp, 0);
+    plan.maxDepth = std::max(plan.maxDepth, lp.maxDepth);
+  }
+  return runPool(b, st, batch.numPaths, plan);
 }
 
 }  // namespace sdb

@@ -10,36 +10,45 @@
 
 namespace sdb {
 
-struct Path;
 struct Vertex;
-struct TraceHit;
 struct GuideTrail;
 
-// A pool entry: the per-path record at a 16-byte boundary, so the stages
-// move it with 128-bit loads and stores (instancing frame: 1,213 Mrays/s
-// against 1,133 at the records' natural 8-byte alignment, 1,158 at 32
-// bytes). The records themselves keep their natural layout, so the
-// megakernel's register and local-memory frames do not grow.
+// A pool entry at a 16-byte boundary, moved with 128-bit loads and stores.
 template <typename T>
 struct __align__(16) PoolSlot {
   T v;
 };
 
-// Device view of the slot pool (one path per slot).
+// Counters of one iteration (cleared on the device before it).
+struct WfCounts {
+  unsigned live;         // rays the iteration traces (its live list's length)
+  unsigned shadow;       // shadow rays it queued
+  unsigned late;         // vertices finished after their shadow ray
+  unsigned traced;       // radiance rays shaded (live without tile padding)
+  unsigned fetchRay, fetchShadow;  // rays taken by the dynamic fetches
+  unsigned pad[2];
+};
+constexpr int kWfGroup = 8;  // iterations launched between two looks at the live count
+
+// Device view of the slot pool (one path per slot). A path's state is three
+// 32-byte records in arrays of their own, so each stage moves whole sectors
+// of what it needs and nothing else:
+//   ray    o.xyz d.xyz, previous BSDF density, flags (specular | medDepth << 1);
+//          of a camera ray the last two words are the random state
+//   sum    L.xyz, sample slot, throughput.xyz, -
+//   rest   previous vertex.xyz, -, random state, medium stack
+// (the depth is the iteration; the random increment is the launch's).
 struct WfPool {
-  PoolSlot<Path>* paths;
-  PoolSlot<Vertex>* verts;
-  PoolSlot<TraceHit>* hits;
-  float4* trs;             // shadow-ray transmittance of the slot's vertex
-  unsigned char* pending;  // 1: the slot's second half is due this iteration
-  int* lists[2];           // live slot lists, ping-pong between iterations
-  int* shadowList;
-  unsigned* counts;        // [0], [1]: list lengths; [2]: shadow-list length;
-                           // [3]: rays the trace stage has fetched
+  float4 *ray, *sum, *rest;   // two float4 each
+  float4* hits;               // two: t, inst, prim | front << 31, u / v, normal.xyz
+  float4* shadowRays;         // two: origin.xyz dir.xyz, tmax, flags
+  float4* shadowTerms;        // the NEE term; for a late vertex its transmittance
+  PoolSlot<Vertex>* verts;    // late vertices (allocated when a launch may have some)
+  int* lists[2];              // live slot lists, ping-pong between iterations
+  int *shadowList, *lateList;
+  WfCounts* counts;           // kWfGroup + 1
   PoolSlot<GuideTrail>* trails;  // guided vertices awaiting their path's end (record passes)
-  unsigned char* jobs;     // serving batches: the job slot of each slot's path
-  int cap;
-  int refillOpen;          // 0: every path of the launch fits the pool at once (no refills)
+  unsigned char* jobs;        // serving batches: the job slot of each slot's path
 };
 
 // Host-owned pool storage, grown on demand.
@@ -47,24 +56,31 @@ struct WfBuffers {
   // One device allocation holds every per-slot array (carved at 256-byte
   // boundaries), so a pool costs one cudaMalloc and one cudaFree.
   DevBuf slab, counts;
-  void *paths = nullptr, *verts = nullptr, *hits = nullptr, *trs = nullptr, *pending = nullptr,
-       *list0 = nullptr, *list1 = nullptr, *shadow = nullptr, *jobs = nullptr;
+  WfPool pool = {};
   DevBuf trails;  // allocated by the first training-record pass
-  unsigned* hostCount = nullptr;   // pinned: the four list counters (from a process-wide free list)
+  unsigned* hostCount = nullptr;   // pinned: counters read back (from a process-wide free list)
   cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};  // stage timing
   int cap = 0;
+  bool late = false;  // the slab holds late vertices
   int trailCap = 0;
-  int gridStart = 0, gridTrace = 0, gridShadeA = 0, gridShadow = 0, gridShadeB = 0;
+  int gridStart = 0, gridTrace = 0, gridShade = 0, gridShadow = 0, gridLate = 0;
   WfBuffers() = default;
   WfBuffers(const WfBuffers&) = delete;
   WfBuffers& operator=(const WfBuffers&) = delete;
   ~WfBuffers();
-  void ensure(int slots);
+  // Room for `slots` paths (fewer when device memory is short); withLate:
+  // with their late vertices.
+  void ensure(int slots, bool withLate);
   void ensureTrails();  // one GuideTrail per slot
 };
 
+// Whether paths of the launch may have late vertices: those whose next draws
+// depend on their shadow ray (flames along it draw a random number) or whose
+// training record needs its radiance.
+bool wfHasLate(const SdLaunch& lp, int guide);
+
 // Device bytes per pool slot.
-size_t wfSlotBytes();
+size_t wfSlotBytes(bool withLate);
 // A pool for the current device: the idle one kept from an earlier session,
 // or a new empty one. wfRelease keeps a finished session's pool for reuse.
 std::unique_ptr<WfBuffers> wfAcquire();
@@ -75,8 +91,9 @@ void wfReleaseIdle();
 // (sundog_set_device_memory_cache; render.cpp).
 bool keepDeviceMemory();
 // Renders lp.numPaths camera paths (counters cleared by the caller) into
-// lp.sampleL; returns the number of kernels launched. Synchronises st once per
-// iteration to read the live-path count. guide: 0, or a combination of
+// lp.sampleL; returns the number of kernels launched. Synchronises st every
+// kWfGroup iterations to read the live-path count, where paths may be longer.
+// guide: 0, or a combination of
 // kGuideSample (draw directions by MIS with the learned guide of lp) and
 // kGuideRecord (keep each path's guided vertices in its slot's trail and turn
 // them into training records when the path ends).
@@ -88,11 +105,11 @@ int wfRender(const SdLaunch& lp, WfBuffers& b, cudaStream_t st, int guide = 0,
 // launch blocks, host memory), and one batch of tile-passes rendered through
 // the pool into batch.sampleL at each path's id (the caller folds them).
 // Returns the kernels launched.
-// maxInstances: the largest instance count among the batch's scenes (picks
-// the shadow-ray kernel, as a render does by its own scene's count).
+// jobs: the same table, for what its scenes need (the shadow-ray kernel, as a
+// render picks it by its own scene's instance count; late vertices).
 struct ServeBatch;
 cudaError_t wfSetJobs(const SdLaunch* table, cudaStream_t st);
-int wfRenderBatch(const ServeBatch& batch, WfBuffers& b, cudaStream_t st, int maxInstances = 0);
+int wfRenderBatch(const ServeBatch& batch, WfBuffers& b, cudaStream_t st, const SdLaunch* jobs);
 
 // Scenes with at least this many instances trace their shadow rays with
 // dynamic fetch (wfShadowFetch), smaller ones one ray per thread (wfShadow).
