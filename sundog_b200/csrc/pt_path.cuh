@@ -179,16 +179,20 @@ struct Vertex {
   bool delta;
 };
 
-// The traced segment's media: absorption of the medium the path is in, then
-// the flames along the segment. t: the hit's distance.
-// (device/programs.cu:374-400)
-__device__ __forceinline__ void crossMedia(const SdLaunch& lp, Path& p, bool hit, float t) {
+// Absorption along the traced segment by the medium the path is in. t: the
+// hit's distance. (device/programs.cu:374-384)
+__device__ __forceinline__ void absorbMedium(const SdLaunch& lp, Path& p, bool hit, float t) {
   if (p.medDepth > 0) {
     int top = min(p.medDepth, 4) - 1;
     float3 sigma = lp.materials[medAt(p.med, top)].absorb;
     if (hmax(sigma) > 0.0f) p.beta *= vexp(-sigma * (hit ? t : 1e4f));
   }
+}
 
+// The traced segment's media: absorption, then the flames along the segment.
+// (device/programs.cu:374-400)
+__device__ __forceinline__ void crossMedia(const SdLaunch& lp, Path& p, bool hit, float t) {
+  absorbMedium(lp, p, hit, t);
   if (lp.numFlames > 0) {
     float3 trans = v3(1.0f);
     float3 Lv = flameMarch(lp.flames, lp.numFlames, p.o, p.d, hit ? t : 1e16f, p.rng, trans);

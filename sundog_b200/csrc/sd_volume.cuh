@@ -305,6 +305,26 @@ SDB_HD bool flameClip(const SdFlame& fl, float3 o, float3 d, float& t0, float& t
   return t0 < t1;
 }
 
+// Whether the segment may enter a flame other than `skip`: flameClip on
+// volumes grown by far more than its rounding errors, so a segment this
+// turns away enters no flame (and draws no jitter).
+SDB_HD bool flamesMayMeet(const SdFlame* fls, int nfl, float3 o, float3 d, float tEnd, int skip) {
+  for (int i = 0; i < nfl; i++) {
+    if (i == skip) continue;
+    SdFlame fl = fls[i];
+    const float reach = fmaxf(fabsf(o.x), fmaxf(fabsf(o.y), fabsf(o.z))) +
+                        fmaxf(fabsf(fl.base.x), fmaxf(fabsf(fl.base.y), fabsf(fl.base.z))) +
+                        fl.height + fl.radius;
+    const float m = 1e-3f * (1.0f + reach);
+    fl.base.y -= m;
+    fl.height += 2.0f * m;
+    fl.radius += m;
+    float t0 = 0.0f, t1 = tEnd * 1.001f;
+    if (flameClip(fl, o, d, t0, t1)) return true;
+  }
+  return false;
+}
+
 // Emission along [1e-4, tEnd] of o + t d through every flame, weighted by the
 // running transmittance; the segment's transmittance is folded into trans.
 // One draw per entered flame. (device/volume.cuh:90-115)

@@ -4,9 +4,10 @@
 //   wfStart        a camera ray in every slot
 //   per iteration (path depth), over the slots in the live list:
 //   wfTraceFetch   trace the radiance ray (traversal only)
-//   wfShade        media, flames, escape, shading, emission, the NEE light
-//                  draw, the BSDF sample and roulette; queues the slot's
-//                  shadow ray with the radiance it would add
+//   wfFlameScan, wfFlame  (scenes with flames) march the rays that may meet one
+//   wfShade        media, escape, shading, emission, the NEE light draw, the
+//                  BSDF sample and roulette; queues the slot's shadow ray
+//                  with the radiance it would add
 //   wfShadow       trace the queued shadow rays (transparent shadows) and
 //                  add that radiance
 //   wfLate         the end of the few vertices that must know their shadow
@@ -65,8 +66,14 @@ constexpr int kRound = (GUIDE & kWfServe) ? kRoundServe : kRoundStage;  // sd_bs
 #endif
 // Resident blocks per SM the stage kernels are compiled for: traversal 8 ->
 // 64 registers, shading 5 -> 102 registers.
+#ifndef SDB_WF_LATE_BLOCKS
+#define SDB_WF_LATE_BLOCKS 5
+#endif
+#ifndef SDB_WF_FLAME_BLOCKS
+#define SDB_WF_FLAME_BLOCKS 5
+#endif
 #ifndef SDB_WF_SHADE_BLOCKS
-#define SDB_WF_SHADE_BLOCKS 5
+#define SDB_WF_SHADE_BLOCKS 3
 #endif
 
 // A 32-byte record in one 256-bit load or store.
@@ -463,10 +470,17 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetc
 // Rays of a tile, shaded together by one block: sorted by what their hit
 // needs (kClass*), so a warp runs one material's code instead of stepping
 // through all of them with a few lanes each.
-constexpr int kTileMax = 8 * kRenderBlock;
+#ifndef SDB_SHADE_THREADS
+#define SDB_SHADE_THREADS 256
+#endif
+#ifndef SDB_SHADE_TILE
+#define SDB_SHADE_TILE 1024
+#endif
+constexpr int kShadeBlock = SDB_SHADE_THREADS;
+constexpr int kTileMax = SDB_SHADE_TILE;
 constexpr int kClasses = 8;       // miss, then 1 + MatKind, then tile padding
 constexpr int kClassNone = 7;
-constexpr int kWarps = kRenderBlock / 32;
+constexpr int kWarps = kShadeBlock / 32;
 
 // Hides a value from the optimiser as a trip through memory does: the two
 // halves of a vertex round the same whether one kernel computes both or the
@@ -510,18 +524,22 @@ __device__ __forceinline__ void storePath(const WfPool& pool, const Path& p, int
 __device__ __forceinline__ unsigned long long join64(float lo, float hi) {
   return (unsigned long long)bitsU(lo) | ((unsigned long long)bitsU(hi) << 32);
 }
+__device__ __forceinline__ void loadSum(const WfPool& pool, int slot, Path& p) {
+  const Rec s = ldRec(pool.sum, slot);
+  p.L = v3(s.a.x, s.a.y, s.a.z);
+  p.slot = __float_as_int(s.a.w);
+  p.beta = v3(s.b.x, s.b.y, s.b.z);
+}
 // The path in `slot` at `depth` (not a camera ray).
 __device__ __forceinline__ void loadPath(const WfPool& pool, const SdLaunch& lp, int slot, int depth,
                                          Path& p) {
-  const Rec r = ldRec(pool.ray, slot), s = ldRec(pool.sum, slot), q = ldRec(pool.rest, slot);
+  const Rec r = ldRec(pool.ray, slot), q = ldRec(pool.rest, slot);
+  loadSum(pool, slot, p);
   p.o = v3(r.a.x, r.a.y, r.a.z);
   p.d = v3(r.a.w, r.b.x, r.b.y);
   p.prevPdf = r.b.z;
   p.specular = (bitsU(r.b.w) & 1u) != 0;
   p.medDepth = (int)(bitsU(r.b.w) >> 1);
-  p.L = v3(s.a.x, s.a.y, s.a.z);
-  p.slot = __float_as_int(s.a.w);
-  p.beta = v3(s.b.x, s.b.y, s.b.z);
   p.prevX = v3(q.a.x, q.a.y, q.a.z);
   p.rng.state = join64(q.b.x, q.b.y);
   p.rng.inc = rngInc(lp);
@@ -562,6 +580,9 @@ __device__ __forceinline__ void loadCamera(const WfPool& pool, const SdLaunch& l
   opaque(p.depth);
 }
 
+constexpr unsigned kPrimMask = 0x3FFFFFFFu;  // hit record: the triangle
+constexpr unsigned kMediaDone = 0x40000000u;  // its segment's media are in the path already
+
 constexpr unsigned kShadowFinal = 1u;  // shadow ray flags: its path has ended
 constexpr unsigned kShadowLate = 2u;   // its vertex is finished by wfLate
 
@@ -576,23 +597,39 @@ __device__ __forceinline__ unsigned shadeRay(const WfPool& pool, int slot, unsig
   else loadPath(pool, lp, slot, depth, p);
   if (CAM && (GUIDE & kGuideRecord)) pool.trails[slot].v.n = 0;
   const Rec hr = ldRec(pool.hits, slot);
+  const bool mediaDone = (bitsU(hr.a.z) & kMediaDone) != 0;
   TraceHit h;
   h.t = hr.a.x;
   h.inst = __float_as_int(hr.a.y);
-  h.prim = (int)(bitsU(hr.a.z) & 0x7FFFFFFFu);
+  h.prim = (int)(bitsU(hr.a.z) & kPrimMask);
   h.front = (bitsU(hr.a.z) >> 31) != 0;
   h.u = hr.a.w;
   h.v = hr.b.x;
   h.nq = v3(hr.b.y, hr.b.z, hr.b.w);
   const bool hit = h.inst >= 0;
-  crossMedia(lp, p, hit, h.t);
+  if (mediaDone) {
+    if (CAM) loadSum(pool, slot, p);
+  } else {
+    absorbMedium(lp, p, hit, h.t);
+    // No flame on the segment: nothing added (but a non-finite throughput
+    // still shows, as it would with flames marched).
+    if (lp.numFlames > 0) addClamped(lp, p, p.beta * 0.0f);
+  }
   Vertex v;
   unsigned long long raysUnused = 0;
   if (!shadeSurface(lp, p, hit, h, raysUnused, v)) {
     finishPath<GUIDE>(p.L, p.slot, slot);
     return 0;
   }
-  const bool late = v.nee && ((GUIDE & kGuideRecord) || (lp.numFlames > 0 && lp.transparentShadows));
+  bool late = false;
+  if (v.nee) {
+    if (GUIDE & kGuideRecord) {
+      late = true;
+    } else if (lp.numFlames > 0 && lp.transparentShadows) {
+      const int skip = v.lightK < lp.numLights ? lp.lights[v.lightK].flameId : -1;
+      late = flamesMayMeet(lp.flames, lp.numFlames, v.so, v.wi, v.tmaxS, skip);
+    }
+  }
   if (v.nee)
     stRec(pool.shadowRays, slot, make_float4(v.so.x, v.so.y, v.so.z, v.wi.x),
           make_float4(v.wi.y, v.wi.z, v.tmaxS, bitsF(late ? kShadowLate : 0u)));
@@ -637,6 +674,50 @@ __device__ __forceinline__ unsigned shadeRay(const WfPool& pool, int slot, unsig
   return 0;
 }
 
+// Lists the traced rays whose segment may meet a flame.
+template <int GUIDE, bool CAM>
+__global__ void __launch_bounds__(kRenderBlock) wfFlameScan(int it) {
+  const WfPool& pool = c_pool;
+  const unsigned n = pool.counts[it].live;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int slot = liveSlot<CAM>(it, i);
+    const float4 h = pool.hits[2 * (size_t)slot];
+    const int inst = __float_as_int(h.y);
+    if (inst == kNoPath) continue;
+    const SdLaunch& lp = slotLaunch<GUIDE>(slot);
+    if (lp.numFlames == 0) continue;
+    const Rec r = ldRec(pool.ray, slot);
+    if (flamesMayMeet(lp.flames, lp.numFlames, v3(r.a.x, r.a.y, r.a.z), v3(r.a.w, r.b.x, r.b.y),
+                      inst >= 0 ? h.x : 1e16f, -1))
+      pool.lateList[appendSlot(&pool.counts[it].flame)] = slot;
+  }
+}
+
+// Their media: absorption and the flame march, ahead of the shading stage.
+// In that stage a few lanes of a warp marched while the others waited; here
+// every lane of a warp marches.
+template <int GUIDE, bool CAM>
+__global__ void __launch_bounds__(kRenderBlock, SDB_WF_FLAME_BLOCKS) wfFlame(
+    int it, int depth, unsigned long long base) {
+  const WfPool& pool = c_pool;
+  const unsigned n = pool.counts[it].flame;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int slot = pool.lateList[i];
+    const SdLaunch& lp = slotLaunch<GUIDE>(slot);
+    Path p;
+    if (CAM) loadCamera<GUIDE>(pool, lp, slot, base + slot, p);
+    else loadPath(pool, lp, slot, depth, p);
+    float4 h = pool.hits[2 * (size_t)slot];
+    crossMedia(lp, p, __float_as_int(h.y) >= 0, h.x);
+    storeSum(pool, p, slot);
+    // The random state: in a camera ray's record, else in the rest.
+    float2* rng = reinterpret_cast<float2*>((CAM ? pool.ray : pool.rest) + 2 * (size_t)slot) +
+                  (CAM ? 3 : 2);
+    *rng = make_float2(bitsF((unsigned)p.rng.state), bitsF((unsigned)(p.rng.state >> 32)));
+    reinterpret_cast<unsigned*>(pool.hits + 2 * (size_t)slot)[2] = bitsU(h.z) | kMediaDone;
+  }
+}
+
 // What the shading of a traced ray runs: 0 a miss, 1 + the kind of the hit
 // face's material, kClassNone for tile padding.
 template <int GUIDE>
@@ -670,7 +751,7 @@ __device__ __forceinline__ unsigned warpPrefix(unsigned v, unsigned& total) {
 // camera rays is kept from bounce to bounce. Small lists take smaller tiles
 // so that every block has one.
 template <int GUIDE, bool CAM>
-__global__ void __launch_bounds__(kRenderBlock, SDB_WF_SHADE_BLOCKS) wfShade(
+__global__ void __launch_bounds__(kShadeBlock, SDB_WF_SHADE_BLOCKS) wfShade(
     int it, int depth, unsigned long long base) {
   __shared__ int sSlot[kTileMax];
   __shared__ unsigned short sKey[kTileMax];    // class << 8 | rank; then the sorted order
@@ -687,18 +768,18 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_SHADE_BLOCKS) wfShade(
   const unsigned n = cnt.live;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned ltMask = (1u << lane) - 1u;
-  const unsigned per = (n + gridDim.x * kRenderBlock - 1) / (gridDim.x * kRenderBlock);
+  const unsigned per = (n + gridDim.x * kShadeBlock - 1) / (gridDim.x * kShadeBlock);
   // Record passes keep the records of the paths that end first: small tiles
   // there, so those are not the misses of large ones.
-  const unsigned most = (GUIDE & kGuideRecord) ? 1u : (unsigned)(kTileMax / kRenderBlock);
+  const unsigned most = (GUIDE & kGuideRecord) ? 1u : (unsigned)(kTileMax / kShadeBlock);
   const int K = (int)min(max(per, 1u), most);
-  const unsigned T = (unsigned)K * kRenderBlock;
+  const unsigned T = (unsigned)K * kShadeBlock;
   for (unsigned t0 = blockIdx.x * T; t0 < n; t0 += gridDim.x * T) {
     // Classes, and each entry's rank among its warp's entries of the class.
-    for (int k = tid; k < kClasses * kGroups; k += kRenderBlock) sCount[k] = 0;
+    for (int k = tid; k < kClasses * kGroups; k += kShadeBlock) sCount[k] = 0;
     __syncthreads();
     for (int k = 0; k < K; k++) {
-      const int e = k * kRenderBlock + tid;
+      const int e = k * kShadeBlock + tid;
       const unsigned i = t0 + e;
       int slot = -1, cls = kClassNone;
       if (i < n) {
@@ -714,34 +795,37 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_SHADE_BLOCKS) wfShade(
     }
     __syncthreads();
     // Prefix over the counts, class by class (two entries per thread).
-    static_assert(kClasses * kGroups == 2 * kRenderBlock, "two counts per thread");
+    static_assert(kClasses * kGroups <= 2 * kShadeBlock, "two counts per thread");
     {
-      const unsigned c0 = sCount[2 * tid], c1 = sCount[2 * tid + 1];
+      const bool in = 2 * tid < kClasses * kGroups;
+      const unsigned c0 = in ? sCount[2 * tid] : 0u, c1 = in ? sCount[2 * tid + 1] : 0u;
       unsigned total;
       const unsigned ex = warpPrefix(c0 + c1, total);
       if (lane == 0) sPart[warp] = total;
       __syncthreads();
       unsigned before = 0;
       for (int w = 0; w < warp; w++) before += sPart[w];
-      sCount[2 * tid] = (unsigned short)(before + ex);
-      sCount[2 * tid + 1] = (unsigned short)(before + ex + c0);
+      if (in) {
+        sCount[2 * tid] = (unsigned short)(before + ex);
+        sCount[2 * tid + 1] = (unsigned short)(before + ex + c0);
+      }
     }
     __syncthreads();
     const int shaded = sCount[kClassNone * kGroups];  // entries that hold a path
     for (int k = 0; k < K; k++) {
-      const int e = k * kRenderBlock + tid;
+      const int e = k * kShadeBlock + tid;
       const unsigned key = sKey[e];
       sOrder[sCount[(key >> 8) * kGroups + (e >> 5)] + (key & 0xFFu)] = (unsigned short)e;
     }
     __syncthreads();
-    for (int j = tid; j < shaded; j += kRenderBlock) {
+    for (int j = tid; j < shaded; j += kShadeBlock) {
       const int e = sOrder[j];
       sFlag[e] = (unsigned char)shadeRay<GUIDE, CAM>(pool, sSlot[e], base + t0 + e, depth);
     }
     __syncthreads();
     // The tile's contributions to the next lists, in its own order.
     for (int k = 0; k < K; k++) {
-      const int e = k * kRenderBlock + tid;
+      const int e = k * kShadeBlock + tid;
       const unsigned f = sFlag[e];
       const unsigned live = __ballot_sync(full, f & 1u), shadow = __ballot_sync(full, f & 2u),
                      late = __ballot_sync(full, f & 4u);
@@ -765,12 +849,12 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_SHADE_BLOCKS) wfShade(
         unsigned long long* rays = (GUIDE & kWfServe) ? c_wbatch.rayCounter : c_wlp.rayCounter;
         atomicAdd(rays, (unsigned long long)shaded + total);
       }
-    } else if (lane == 0) {
+    } else if (warp == 3 && lane == 0) {
       atomicAdd(&cnt.traced, (unsigned)shaded);
     }
     __syncthreads();
     for (int k = 0; k < K; k++) {
-      const int e = k * kRenderBlock + tid;
+      const int e = k * kShadeBlock + tid;
       const unsigned f = sFlag[e];
       const unsigned live = __ballot_sync(full, f & 1u), shadow = __ballot_sync(full, f & 2u),
                      late = __ballot_sync(full, f & 4u);
@@ -917,7 +1001,7 @@ __global__ void wfShadowFetch(int, int) {}
 // NEE contribution, the BSDF sample, roulette. GUIDE & kGuideRecord: the
 // guided vertex joins the slot's trail.
 template <int GUIDE>
-__global__ void __launch_bounds__(kRenderBlock, SDB_WF_SHADE_BLOCKS) wfLate(int it, int depth) {
+__global__ void __launch_bounds__(kRenderBlock, SDB_WF_LATE_BLOCKS) wfLate(int it, int depth) {
   const WfPool& pool = c_pool;
   const unsigned n = pool.counts[it].late;
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -953,11 +1037,11 @@ static_assert(kWfGroup % 2 == 0, "lists ping-pong back to their place");
 // ---- host ---------------------------------------------------------------------
 
 template <typename K>
-static int gridFor(K kernel) {
+static int gridFor(K kernel, int block = kRenderBlock) {
   int dev = 0, sms = 0, perSm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, kRenderBlock, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, block, 0);
   return sms * (perSm < 1 ? 1 : perSm);
 }
 
@@ -1010,10 +1094,11 @@ void WfBuffers::ensure(int slots, bool withLate) {
   cap = slots;
   late = withLate;
   gridTrace = gridFor(wfTraceFetch<false, false>);
-  gridShade = gridFor(wfShade<0, false>);
+  gridShade = gridFor(wfShade<0, false>, kShadeBlock);
   gridShadow = gridFor(wfShadow<0>);
   gridLate = gridFor(wfLate<0>);
   gridStart = gridFor(wfStart<0>);
+  gridFlame = gridFor(wfFlame<0, false>);
 }
 
 void WfBuffers::ensureTrails() {
@@ -1072,6 +1157,7 @@ struct WfPlan {
   bool shadowFetch;   // the shadow-ray kernel (kShadowFetchInstances)
   bool lights;        // any NEE strategy: shadow rays can exist
   bool late;          // late vertices can exist
+  bool flames;        // some scene has flames
   int maxDepth;
 };
 
@@ -1084,7 +1170,12 @@ static int wfIteration(const WfBuffers& b, cudaStream_t st, int it, int depth,
   if (timed) cudaEventRecord(b.ev[1], st);
   wfTraceFetch<(GUIDE & kWfServe) != 0, CAM><<<b.gridTrace, kRenderBlock, 0, st>>>(it);
   if (timed) cudaEventRecord(b.ev[2], st);
-  wfShade<GUIDE, CAM><<<b.gridShade, kRenderBlock, 0, st>>>(it, depth, base);
+  if (plan.flames) {
+    wfFlameScan<GUIDE, CAM><<<b.gridStart, kRenderBlock, 0, st>>>(it);
+    wfFlame<GUIDE, CAM><<<b.gridFlame, kRenderBlock, 0, st>>>(it, depth, base);
+    launches += 2;
+  }
+  wfShade<GUIDE, CAM><<<b.gridShade, kShadeBlock, 0, st>>>(it, depth, base);
   if (timed) cudaEventRecord(b.ev[3], st);
   if (plan.lights) {
     if (plan.shadowFetch && !SDB_WIDE_BVH)
@@ -1201,7 +1292,7 @@ int wfRender(const SdLaunch& lp, WfBuffers& b, cudaStream_t st, int guide, WfSta
             "wavefront launch block");
   const WfPlan plan = {guide, lp.numInstances >= kShadowFetchInstances,
                        lp.numLights > 0 || lp.bgKind == BG_ENVMAP, wfHasLate(lp, guide),
-                       lp.maxDepth};
+                       lp.numFlames > 0, lp.maxDepth};
   return runPool(b, st, lp.numPaths, plan, times);
 }
 
@@ -1213,12 +1304,13 @@ cudaError_t wfSetJobs(const SdLaunch* table, cudaStream_t st) {
 int wfRenderBatch(const ServeBatch& batch, WfBuffers& b, cudaStream_t st, const SdLaunch* jobs) {
   cudaCheck(cudaMemcpyToSymbolAsync(c_wbatch, &batch, sizeof batch, 0, cudaMemcpyHostToDevice, st),
             "wavefront batch");
-  WfPlan plan = {kWfServe, false, false, false, 0};
+  WfPlan plan = {kWfServe, false, false, false, false, 0};
   for (int k = 0; k < kMaxServeJobs; k++) {  // unused slots are zero
     const SdLaunch& lp = jobs[k];
     plan.shadowFetch = plan.shadowFetch || lp.numInstances >= kShadowFetchInstances;
     plan.lights = plan.lights || lp.numLights > 0 || (lp.width > 0 && lp.bgKind == BG_ENVMAP);
     plan.late = plan.late || wfHasLate(lp, 0);
+    plan.flames = plan.flames || lp.numFlames > 0;
     plan.maxDepth = std::max(plan.maxDepth, lp.maxDepth);
   }
   return runPool(b, st, batch.numPaths, plan);

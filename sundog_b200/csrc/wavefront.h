@@ -26,7 +26,8 @@ struct WfCounts {
   unsigned late;         // vertices finished after their shadow ray
   unsigned traced;       // radiance rays shaded (live without tile padding)
   unsigned fetchRay, fetchShadow;  // rays taken by the dynamic fetches
-  unsigned pad[2];
+  unsigned flame;        // rays that may meet a flame
+  unsigned pad;
 };
 constexpr int kWfGroup = 8;  // iterations launched between two looks at the live count
 
@@ -40,12 +41,13 @@ constexpr int kWfGroup = 8;  // iterations launched between two looks at the liv
 // (the depth is the iteration; the random increment is the launch's).
 struct WfPool {
   float4 *ray, *sum, *rest;   // two float4 each
-  float4* hits;               // two: t, inst, prim | front << 31, u / v, normal.xyz
+  float4* hits;               // two: t, inst, prim | media << 30 | front << 31, u / v, normal.xyz
   float4* shadowRays;         // two: origin.xyz dir.xyz, tmax, flags
   float4* shadowTerms;        // the NEE term; for a late vertex its transmittance
   PoolSlot<Vertex>* verts;    // late vertices (allocated when a launch may have some)
   int* lists[2];              // live slot lists, ping-pong between iterations
-  int *shadowList, *lateList;
+  int *shadowList;
+  int *lateList;              // late vertices; before shading, the rays that may meet a flame
   WfCounts* counts;           // kWfGroup + 1
   PoolSlot<GuideTrail>* trails;  // guided vertices awaiting their path's end (record passes)
   unsigned char* jobs;        // serving batches: the job slot of each slot's path
@@ -63,7 +65,8 @@ struct WfBuffers {
   int cap = 0;
   bool late = false;  // the slab holds late vertices
   int trailCap = 0;
-  int gridStart = 0, gridTrace = 0, gridShade = 0, gridShadow = 0, gridLate = 0;
+  int gridStart = 0, gridTrace = 0, gridShade = 0, gridShadow = 0, gridLate = 0,
+      gridFlame = 0;
   WfBuffers() = default;
   WfBuffers(const WfBuffers&) = delete;
   WfBuffers& operator=(const WfBuffers&) = delete;
