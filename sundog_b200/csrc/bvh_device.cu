@@ -787,16 +787,8 @@ __device__ __forceinline__ void binChild(const BvhNode& n, int side, float3& lo,
 }
 
 __device__ __forceinline__ void setSlot(Bvh4Node& q, int k, float3 lo, float3 hi, int link) {
-  float4& xy = k == 0 ? q.xy0 : k == 1 ? q.xy1 : k == 2 ? q.xy2 : q.xy3;
-  float4& zz = k < 2 ? q.zz01 : q.zz23;
-  xy = make_float4(lo.x, hi.x, lo.y, hi.y);
-  if (k & 1) {
-    zz.z = lo.z;
-    zz.w = hi.z;
-  } else {
-    zz.x = lo.z;
-    zz.y = hi.z;
-  }
+  const float planes[6] = {lo.x, hi.x, lo.y, hi.y, lo.z, hi.z};
+  for (int a = 0; a < 6; a++) reinterpret_cast<float*>(&q.plane[a])[k] = planes[a];
   reinterpret_cast<int*>(&q.link)[k] = link;
 }
 

@@ -153,6 +153,19 @@ __device__ __forceinline__ void boxPair(const BvhNode& nd, float3 oi, float3 id,
   tb = n1;
 }
 
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  float2 o;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(o.x), "=f"(o.y) : "l"(r));
+  return o;
+}
+
 // Orders (d, l) pairs: the smaller distance first, ties keep their order.
 __device__ __forceinline__ void cswap(float& da, int& la, float& db, int& lb) {
   if (db < da) {
@@ -595,31 +608,34 @@ __device__ __forceinline__ int binTravStep(BinTrav& t, TravStack& stack, const S
   if (t.cur >= 0) {
     // Four child boxes; the nearest hit child next, the other hits pushed
     // (farthest first for radiance rays).
-    const float4* np = reinterpret_cast<const float4*>(lp.nodes4 + t.cur);
     if (COUNT) cnt->boxTests += 4;
     const float inf = __int_as_float(0x7f800000);
     float d0, d1, d2, d3;
-    {
-      BvhNode pr;
-      pr.xy0 = __ldg(np);
-      pr.xy1 = __ldg(np + 1);
-      pr.zz = __ldg(np + 2);
-      bool h0, h1;
-      boxPair(pr, t.oi, t.id, tmin, t.tmax, d0, d1, h0, h1);
-      d0 = h0 ? d0 : inf;
-      d1 = h1 ? d1 : inf;
-    }
-    {
-      BvhNode pr;
-      pr.xy0 = __ldg(np + 3);
-      pr.xy1 = __ldg(np + 4);
-      pr.zz = __ldg(np + 5);
-      bool h2, h3;
-      boxPair(pr, t.oi, t.id, tmin, t.tmax, d2, d3, h2, h3);
-      d2 = h2 ? d2 : inf;
-      d3 = h3 ? d3 : inf;
-    }
+    const int sx = (int)(__float_as_uint(t.id.x) >> 31), sy = (int)(__float_as_uint(t.id.y) >> 31),
+              sz = (int)(__float_as_uint(t.id.z) >> 31);
+    const float4* np = reinterpret_cast<const float4*>(lp.nodes4 + t.cur);
+    const float4 nx = __ldg(np + sx), ny = __ldg(np + 2 + sy), nz = __ldg(np + 4 + sz);
+    const float4 fx = __ldg(np + (sx ^ 1)), fy = __ldg(np + 2 + (sy ^ 1)), fz = __ldg(np + 4 + (sz ^ 1));
     const int4 lk = __ldg(reinterpret_cast<const int4*>(np + 6));
+    const float kFar = 1.00000024f;
+    const unsigned long long ix = pack2(t.id.x, t.id.x), iy = pack2(t.id.y, t.id.y), iz = pack2(t.id.z, t.id.z);
+    const unsigned long long mx = pack2(-t.oi.x, -t.oi.x), my = pack2(-t.oi.y, -t.oi.y), mz = pack2(-t.oi.z, -t.oi.z);
+    const float2 nx0 = fma2(pack2(nx.x, nx.y), ix, mx), nx1 = fma2(pack2(nx.z, nx.w), ix, mx);
+    const float2 ny0 = fma2(pack2(ny.x, ny.y), iy, my), ny1 = fma2(pack2(ny.z, ny.w), iy, my);
+    const float2 nz0 = fma2(pack2(nz.x, nz.y), iz, mz), nz1 = fma2(pack2(nz.z, nz.w), iz, mz);
+    const float2 fx0 = fma2(pack2(fx.x, fx.y), ix, mx), fx1 = fma2(pack2(fx.z, fx.w), ix, mx);
+    const float2 fy0 = fma2(pack2(fy.x, fy.y), iy, my), fy1 = fma2(pack2(fy.z, fy.w), iy, my);
+    const float2 fz0 = fma2(pack2(fz.x, fz.y), iz, mz), fz1 = fma2(pack2(fz.z, fz.w), iz, mz);
+#define BOXT(D, NX, NY, NZ, FX, FY, FZ)                                               \
+  {                                                                                   \
+    const float n = fmaxf(fmaxf(NX, NY), fmaxf(NZ, tmin));                            \
+    const float f = fminf(fminf(FX, FY), fminf(FZ, t.tmax)) * kFar;                   \
+    D = n <= f ? n : inf;                                                             \
+  }
+    BOXT(d0, nx0.x, ny0.x, nz0.x, fx0.x, fy0.x, fz0.x)
+    BOXT(d1, nx0.y, ny0.y, nz0.y, fx0.y, fy0.y, fz0.y)
+    BOXT(d2, nx1.x, ny1.x, nz1.x, fx1.x, fy1.x, fz1.x)
+    BOXT(d3, nx1.y, ny1.y, nz1.y, fx1.y, fy1.y, fz1.y)
     int l0 = lk.x, l1 = lk.y, l2 = lk.z, l3 = lk.w;
     // The nearest hit child first (three exchanges put the minimum in slot
     // 0); radiance rays also order the rest for front-to-back pops, shadow

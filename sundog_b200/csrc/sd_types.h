@@ -144,9 +144,8 @@ struct __align__(16) BvhNode {
 // yet loaded), then the four links (inner node index >= 0, leaf code < 0 as
 // in BvhNode). An unused slot has the far point (3e30, 3e30, 3e30) as its
 // box, which no ray reaches within its tmax.
-struct __align__(16) Bvh4Node {
-  float4 xy0, xy1, zz01;  // children 0 and 1: lo.x hi.x lo.y hi.y / ... / lo.z hi.z lo.z hi.z
-  float4 xy2, xy3, zz23;  // children 2 and 3
+struct __align__(128) Bvh4Node {
+  float4 plane[6];  // lo.x hi.x lo.y hi.y lo.z hi.z of children 0-3
   int4 link;
   int4 pad;
 };
