@@ -27,6 +27,7 @@
 //    before starting any stream capture.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include <stdexcept>
@@ -35,6 +36,7 @@
 #include "abi_util.h"
 #include "pt_path.cuh"
 #include "render_session.h"
+#include "wavefront.h"
 
 namespace sdb {
 
@@ -74,7 +76,7 @@ __device__ __forceinline__ unsigned long long fullFrameId(const SdLaunch& lp, in
   return (unsigned long long)rem * lp.sppThisLaunch + sLocal;
 }
 
-__global__ void __launch_bounds__(kRenderBlock) ptTileNoAlloc() {
+__global__ void __launch_bounds__(kRenderBlock) ptTileNoAlloc(int lanes) {
   const SdLaunch& lp = g_tileLp;
   const TileSpec& t = g_tile;
   const unsigned full = 0xFFFFFFFFu;
@@ -82,8 +84,10 @@ __global__ void __launch_bounds__(kRenderBlock) ptTileNoAlloc() {
   unsigned long long rays = 0;
   const int npt = t.w * t.h;
   const long long total = (long long)npt * t.sampleCount;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
+  // Each warp takes `lanes` consecutive path indices per round.
+  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long warps = (long long)gridDim.x * blockDim.x >> 5;
+  for (long long i = warp * lanes + lane; lane < lanes && i < total; i += warps * lanes) {
     // The samples of a pixel are consecutive (total is at most kTileSlots).
     int rem = (int)i / t.sampleCount;
     int sLocal = (int)i - rem * t.sampleCount;
@@ -194,8 +198,19 @@ extern "C" int sundog_session_render_tile_noalloc(sundog_session* sh, int x0, in
   ptTileSetup<<<1, 1, 0, st>>>(lp, t);
   cudaCheck(cudaGetLastError(), "noalloc set-up launch");
   long long total = (long long)w * h * sample_count;
-  int grid = (int)((total + kRenderBlock - 1) / kRenderBlock);
-  ptTileNoAlloc<<<grid, kRenderBlock, 0, st>>>();
+  // A small tile is bound by its longest warp, so its paths are spread over
+  // more warps than they fill: over 16 per SM where walks or flame marches are
+  // long (volumes 18x18 at 6 samples 157 -> 113 us, instancing 40x40 at 9
+  // 362 -> 311; at 2 per SM 128 and 376), over one per SM where they are short
+  // (Cornell 8x8 at 1 sample 92 -> 58 us; 32x32 at 4 takes 111 us in full
+  // warps, 117 over 2 per SM and 120 over 16: paths in step share their
+  // instruction fetches).
+  const bool uneven = lp.numInstances >= kShadowFetchInstances || lp.numFlames > 0;
+  const long long spread = 148 * (uneven ? 16 : 1);
+  const int lanes = (int)std::min<long long>(32, (total + spread - 1) / spread);
+  const long long warps = (total + lanes - 1) / lanes;
+  int grid = (int)((warps * 32 + kRenderBlock - 1) / kRenderBlock);
+  ptTileNoAlloc<<<grid, kRenderBlock, 0, st>>>(lanes);
   cudaCheck(cudaGetLastError(), "noalloc render launch");
   ptTileFold<<<(w * h + 255) / 256, 256, 0, st>>>();
   cudaCheck(cudaGetLastError(), "noalloc fold launch");
