@@ -569,6 +569,7 @@ __device__ __forceinline__ void binTravStart(BinTrav& t, const SdLaunch& lp, flo
 constexpr int kTravDone = 0;      // every node visited
 constexpr int kTravMore = 1;      // more steps to take
 constexpr int kTravOccluded = 2;  // shadow rays: an opaque crossing
+constexpr int kTravLeaf = 3;      // more triangles of the leaf to test
 
 // Takes the next stack entry into t.cur, the step that ends a node or a leaf
 // with nothing left to descend into (done in that same step, so no loop
@@ -591,6 +592,174 @@ __device__ __forceinline__ int binTravPop(BinTrav& t, TravStack& stack, Sink& si
   return kTravMore;
 }
 
+// A TLAS leaf: one instance's quadric roots, or entry into its BLAS.
+template <bool SHADOW, bool COUNT, class Sink>
+__device__ __forceinline__ int binTravInstance(BinTrav& t, TravStack& stack, const SdLaunch& lp,
+                                               Sink& sink, float& trProd, float3& tau,
+                                               TraceCount* cnt) {
+  const float tmin = 0.0f;
+  const int start = ~t.cur >> 3;
+  // TLAS leaves hold exactly one instance; ro, rd are the world ray here.
+  const SdInstance& in = lp.inst[start];
+  float3 o2 = xfPoint(in.w2o, t.ro), d2 = xfVec(in.w2o, t.rd);
+  if (in.kind == GK_MESH) {
+    if (COUNT) cnt->blasEntries++;
+    // Always room: the scene build bounds TLAS + BLAS depth by the stack.
+    if (t.sp < kStackSize) {
+      stack[t.sp++] = kToTlas;
+      t.inBlas = true;
+      t.curInst = start;
+      t.ro = o2;
+      t.rd = d2;
+      t.id = v3(safeInv(d2.x), safeInv(d2.y), safeInv(d2.z));
+      t.oi = o2 * t.id;
+      t.wr = wtSetup(d2);
+      t.cur = lp.meshes[in.mesh].root;
+      return kTravMore;
+    }
+    return binTravPop(t, stack, sink);
+  }
+  if (COUNT) cnt->quadTests++;
+  QHits qh = hitQuadric(in.kind, o2, d2, tmin, t.tmax);
+  for (int k = 0; k < qh.n; k++) {
+    const QHit& q = qh.h[k];
+    if (q.t >= t.tmax) continue;
+    bool front = dot(q.n, d2) < 0.0f;
+    if ((in.flags & kInstMasked) && !faceAccepts(lp, in, front, q.u, q.v)) continue;
+    if (SHADOW) {
+      if (!(in.flags & kInstTransmissive)) return kTravOccluded;
+      uint16_t mid = front ? (uint16_t)(in.mats & 0xFFFF) : (uint16_t)(in.mats >> 16);
+      ShadePt spt = quadShade(in, q.n, q.u, q.v, sink.worldDir());
+      if (!shadowCross(lp, spt, mid, q.t, sink.worldDir(), trProd, tau)) return kTravOccluded;
+    } else {
+      t.tmax = q.t;
+      sink.hit(q.t, start, 0, q.u, q.v, q.n, front);
+    }
+  }
+  return binTravPop(t, stack, sink);
+}
+
+// One triangle of the current BLAS leaf, in object space of curInst. Returns
+// kTravLeaf while the leaf holds more (cur then names the rest), else pops.
+template <bool SHADOW, bool COUNT, class Sink>
+__device__ __forceinline__ int binTravTriangle(BinTrav& t, TravStack& stack, const SdLaunch& lp,
+                                               Sink& sink, float& trProd, float3& tau,
+                                               TraceCount* cnt) {
+  const float tmin = 0.0f;
+  const int code = ~t.cur;
+  const float4* tp = lp.tris + 3 * (size_t)(code >> 3);
+  float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
+  if (COUNT) cnt->triTests++;
+  float tt, b1, b2;
+  float3 p0 = v3(a.x, a.y, a.z), p1 = v3(b.x, b.y, b.z), p2 = v3(c.x, c.y, c.z);
+  if (wtHit(t.wr, t.ro, p0, p1, p2, tmin, t.tmax, tt, b1, b2)) {
+    const int prim = __float_as_int(a.w);
+    const SdInstance& in = lp.inst[t.curInst];
+    if (!(in.flags & (kInstMasked | kInstTransmissive))) {
+      if (SHADOW) return kTravOccluded;
+      t.tmax = tt;
+      sink.hit(tt, t.curInst, prim, b1, b2, v3(0.0f), dot(cross(p1 - p0, p2 - p0), t.rd) < 0.0f);
+    } else {
+      ShadePt spt = triShade(lp, in, prim, b1, b2, sink.worldDir());
+      if (!(in.flags & kInstMasked) || faceAccepts(lp, in, spt.front, spt.u, spt.v)) {
+        if (SHADOW) {
+          if (!(in.flags & kInstTransmissive)) return kTravOccluded;
+          uint16_t mid = spt.front ? (uint16_t)(in.mats & 0xFFFF) : (uint16_t)(in.mats >> 16);
+          if (!shadowCross(lp, spt, mid, tt, sink.worldDir(), trProd, tau)) return kTravOccluded;
+        } else {
+          t.tmax = tt;
+          sink.hit(tt, t.curInst, prim, b1, b2, v3(0.0f), spt.front);
+        }
+      }
+    }
+  }
+  if (code & 7) {  // the next triangle of the leaf, one fewer left
+    t.cur = ~(code + 7);
+    return kTravLeaf;
+  }
+  return binTravPop(t, stack, sink);
+}
+
+// A node visit: the boxes of its children.
+template <bool SHADOW, bool COUNT, class Sink>
+__device__ __forceinline__ int binTravNode(BinTrav& t, TravStack& stack, const SdLaunch& lp,
+                                           Sink& sink, TraceCount* cnt) {
+  const float tmin = 0.0f;
+#if SDB_BVH4
+  // Four child boxes; the nearest hit child next, the other hits pushed
+  // (farthest first for radiance rays).
+  if (COUNT) cnt->boxTests += 4;
+  const float inf = __int_as_float(0x7f800000);
+  float d0, d1, d2, d3;
+  const int sx = (int)(__float_as_uint(t.id.x) >> 31), sy = (int)(__float_as_uint(t.id.y) >> 31),
+            sz = (int)(__float_as_uint(t.id.z) >> 31);
+  const float4* np = reinterpret_cast<const float4*>(lp.nodes4 + t.cur);
+  const float4 nx = __ldg(np + sx), ny = __ldg(np + 2 + sy), nz = __ldg(np + 4 + sz);
+  const float4 fx = __ldg(np + (sx ^ 1)), fy = __ldg(np + 2 + (sy ^ 1)), fz = __ldg(np + 4 + (sz ^ 1));
+  const int4 lk = __ldg(reinterpret_cast<const int4*>(np + 6));
+  const float kFar = 1.00000024f;
+  const unsigned long long ix = pack2(t.id.x, t.id.x), iy = pack2(t.id.y, t.id.y), iz = pack2(t.id.z, t.id.z);
+  const unsigned long long mx = pack2(-t.oi.x, -t.oi.x), my = pack2(-t.oi.y, -t.oi.y), mz = pack2(-t.oi.z, -t.oi.z);
+  const float2 nx0 = fma2(pack2(nx.x, nx.y), ix, mx), nx1 = fma2(pack2(nx.z, nx.w), ix, mx);
+  const float2 ny0 = fma2(pack2(ny.x, ny.y), iy, my), ny1 = fma2(pack2(ny.z, ny.w), iy, my);
+  const float2 nz0 = fma2(pack2(nz.x, nz.y), iz, mz), nz1 = fma2(pack2(nz.z, nz.w), iz, mz);
+  const float2 fx0 = fma2(pack2(fx.x, fx.y), ix, mx), fx1 = fma2(pack2(fx.z, fx.w), ix, mx);
+  const float2 fy0 = fma2(pack2(fy.x, fy.y), iy, my), fy1 = fma2(pack2(fy.z, fy.w), iy, my);
+  const float2 fz0 = fma2(pack2(fz.x, fz.y), iz, mz), fz1 = fma2(pack2(fz.z, fz.w), iz, mz);
+#define BOXT(D, NX, NY, NZ, FX, FY, FZ)                                               \
+  {                                                                                   \
+  const float n = fmaxf(fmaxf(NX, NY), fmaxf(NZ, tmin));                            \
+  const float f = fminf(fminf(FX, FY), fminf(FZ, t.tmax)) * kFar;                   \
+  D = n <= f ? n : inf;                                                             \
+  }
+  BOXT(d0, nx0.x, ny0.x, nz0.x, fx0.x, fy0.x, fz0.x)
+  BOXT(d1, nx0.y, ny0.y, nz0.y, fx0.y, fy0.y, fz0.y)
+  BOXT(d2, nx1.x, ny1.x, nz1.x, fx1.x, fy1.x, fz1.x)
+  BOXT(d3, nx1.y, ny1.y, nz1.y, fx1.y, fy1.y, fz1.y)
+  int l0 = lk.x, l1 = lk.y, l2 = lk.z, l3 = lk.w;
+  // The nearest hit child first (three exchanges put the minimum in slot
+  // 0); radiance rays also order the rest for front-to-back pops, shadow
+  // rays, which stop at any opaque hit, take them as found (shadow stage
+  // 119.0 -> 115.6 ms on config 2, 22.9 -> 22.5 ms on config 1).
+  cswap(d0, l0, d1, l1);
+  cswap(d2, l2, d3, l3);
+  cswap(d0, l0, d2, l2);
+  if (!SHADOW) {
+    cswap(d1, l1, d3, l3);
+    cswap(d1, l1, d2, l2);
+  }
+  if (!(d0 < inf)) return binTravPop(t, stack, sink);
+  // Always room: the scene build bounds the tree depths by the stack.
+  if (d3 < inf && t.sp < kStackSize) stack[t.sp++] = l3;
+  if (d2 < inf && t.sp < kStackSize) stack[t.sp++] = l2;
+  if (d1 < inf && t.sp < kStackSize) stack[t.sp++] = l1;
+  t.cur = l0;
+  return kTravMore;
+#else
+  BvhNode nd = loadNode(lp.nodes, t.cur);
+  if (COUNT) cnt->boxTests += 2;
+  float ta, tb;
+  bool ha, hb;
+  boxPair(nd, t.oi, t.id, tmin, t.tmax, ta, tb, ha, hb);
+  if (ha && hb) {
+    int first = nd.link.x, second = nd.link.y;
+    if (tb < ta) {
+      first = nd.link.y;
+      second = nd.link.x;
+    }
+    if (t.sp < kStackSize) stack[t.sp++] = second;
+    t.cur = first;
+  } else if (ha) {
+    t.cur = nd.link.x;
+  } else if (hb) {
+    t.cur = nd.link.y;
+  } else {
+    return binTravPop(t, stack, sink);
+  }
+  return kTravMore;
+#endif
+}
+
 // One action of the walk. The sink receives what the walk finds and owns
 // the world ray: sink.world(ro, rd) restores it when the walk leaves a BLAS,
 // sink.worldDir() is the world direction for shading a candidate, and
@@ -602,157 +771,15 @@ template <bool SHADOW, bool COUNT, class Sink>
 __device__ __forceinline__ int binTravStep(BinTrav& t, TravStack& stack, const SdLaunch& lp,
                                            Sink& sink, float& trProd, float3& tau,
                                            TraceCount* cnt) {
-  const float tmin = 0.0f;
   if (COUNT) countWarp(cnt, cnt->travIters, cnt->travLanes);
-#if SDB_BVH4
-  if (t.cur >= 0) {
-    // Four child boxes; the nearest hit child next, the other hits pushed
-    // (farthest first for radiance rays).
-    if (COUNT) cnt->boxTests += 4;
-    const float inf = __int_as_float(0x7f800000);
-    float d0, d1, d2, d3;
-    const int sx = (int)(__float_as_uint(t.id.x) >> 31), sy = (int)(__float_as_uint(t.id.y) >> 31),
-              sz = (int)(__float_as_uint(t.id.z) >> 31);
-    const float4* np = reinterpret_cast<const float4*>(lp.nodes4 + t.cur);
-    const float4 nx = __ldg(np + sx), ny = __ldg(np + 2 + sy), nz = __ldg(np + 4 + sz);
-    const float4 fx = __ldg(np + (sx ^ 1)), fy = __ldg(np + 2 + (sy ^ 1)), fz = __ldg(np + 4 + (sz ^ 1));
-    const int4 lk = __ldg(reinterpret_cast<const int4*>(np + 6));
-    const float kFar = 1.00000024f;
-    const unsigned long long ix = pack2(t.id.x, t.id.x), iy = pack2(t.id.y, t.id.y), iz = pack2(t.id.z, t.id.z);
-    const unsigned long long mx = pack2(-t.oi.x, -t.oi.x), my = pack2(-t.oi.y, -t.oi.y), mz = pack2(-t.oi.z, -t.oi.z);
-    const float2 nx0 = fma2(pack2(nx.x, nx.y), ix, mx), nx1 = fma2(pack2(nx.z, nx.w), ix, mx);
-    const float2 ny0 = fma2(pack2(ny.x, ny.y), iy, my), ny1 = fma2(pack2(ny.z, ny.w), iy, my);
-    const float2 nz0 = fma2(pack2(nz.x, nz.y), iz, mz), nz1 = fma2(pack2(nz.z, nz.w), iz, mz);
-    const float2 fx0 = fma2(pack2(fx.x, fx.y), ix, mx), fx1 = fma2(pack2(fx.z, fx.w), ix, mx);
-    const float2 fy0 = fma2(pack2(fy.x, fy.y), iy, my), fy1 = fma2(pack2(fy.z, fy.w), iy, my);
-    const float2 fz0 = fma2(pack2(fz.x, fz.y), iz, mz), fz1 = fma2(pack2(fz.z, fz.w), iz, mz);
-#define BOXT(D, NX, NY, NZ, FX, FY, FZ)                                               \
-  {                                                                                   \
-    const float n = fmaxf(fmaxf(NX, NY), fmaxf(NZ, tmin));                            \
-    const float f = fminf(fminf(FX, FY), fminf(FZ, t.tmax)) * kFar;                   \
-    D = n <= f ? n : inf;                                                             \
-  }
-    BOXT(d0, nx0.x, ny0.x, nz0.x, fx0.x, fy0.x, fz0.x)
-    BOXT(d1, nx0.y, ny0.y, nz0.y, fx0.y, fy0.y, fz0.y)
-    BOXT(d2, nx1.x, ny1.x, nz1.x, fx1.x, fy1.x, fz1.x)
-    BOXT(d3, nx1.y, ny1.y, nz1.y, fx1.y, fy1.y, fz1.y)
-    int l0 = lk.x, l1 = lk.y, l2 = lk.z, l3 = lk.w;
-    // The nearest hit child first (three exchanges put the minimum in slot
-    // 0); radiance rays also order the rest for front-to-back pops, shadow
-    // rays, which stop at any opaque hit, take them as found (shadow stage
-    // 119.0 -> 115.6 ms on config 2, 22.9 -> 22.5 ms on config 1).
-    cswap(d0, l0, d1, l1);
-    cswap(d2, l2, d3, l3);
-    cswap(d0, l0, d2, l2);
-    if (!SHADOW) {
-      cswap(d1, l1, d3, l3);
-      cswap(d1, l1, d2, l2);
-    }
-    if (!(d0 < inf)) return binTravPop(t, stack, sink);
-    // Always room: the scene build bounds the tree depths by the stack.
-    if (d3 < inf && t.sp < kStackSize) stack[t.sp++] = l3;
-    if (d2 < inf && t.sp < kStackSize) stack[t.sp++] = l2;
-    if (d1 < inf && t.sp < kStackSize) stack[t.sp++] = l1;
-    t.cur = l0;
-    return kTravMore;
-  }
-#endif
-  if (t.cur >= 0) {
-    BvhNode nd = loadNode(lp.nodes, t.cur);
-    if (COUNT) cnt->boxTests += 2;
-    float ta, tb;
-    bool ha, hb;
-    boxPair(nd, t.oi, t.id, tmin, t.tmax, ta, tb, ha, hb);
-    if (ha && hb) {
-      int first = nd.link.x, second = nd.link.y;
-      if (tb < ta) {
-        first = nd.link.y;
-        second = nd.link.x;
-      }
-      if (t.sp < kStackSize) stack[t.sp++] = second;
-      t.cur = first;
-    } else if (ha) {
-      t.cur = nd.link.x;
-    } else if (hb) {
-      t.cur = nd.link.y;
-    } else {
-      return binTravPop(t, stack, sink);
-    }
-    return kTravMore;
-  }
+  if (t.cur >= 0) return binTravNode<SHADOW, COUNT>(t, stack, lp, sink, cnt);
   if (t.cur == kPop) return binTravPop(t, stack, sink);  // a walk with no TLAS
   // Leaf: ~cur = start << 3 | (count - 1).
-  const int code = ~t.cur;
-  const int start = code >> 3;
-  const int count = (code & 7) + 1;
-  if (!t.inBlas) {
-    // TLAS leaves hold exactly one instance; ro, rd are the world ray here.
-    const SdInstance& in = lp.inst[start];
-    float3 o2 = xfPoint(in.w2o, t.ro), d2 = xfVec(in.w2o, t.rd);
-    if (in.kind == GK_MESH) {
-      if (COUNT) cnt->blasEntries++;
-      // Always room: the scene build bounds TLAS + BLAS depth by the stack.
-      if (t.sp < kStackSize) {
-        stack[t.sp++] = kToTlas;
-        t.inBlas = true;
-        t.curInst = start;
-        t.ro = o2;
-        t.rd = d2;
-        t.id = v3(safeInv(d2.x), safeInv(d2.y), safeInv(d2.z));
-        t.oi = o2 * t.id;
-        t.wr = wtSetup(d2);
-        t.cur = lp.meshes[in.mesh].root;
-        return kTravMore;
-      }
-      return binTravPop(t, stack, sink);
-    }
-    if (COUNT) cnt->quadTests++;
-    QHits qh = hitQuadric(in.kind, o2, d2, tmin, t.tmax);
-    for (int k = 0; k < qh.n; k++) {
-      const QHit& q = qh.h[k];
-      if (q.t >= t.tmax) continue;
-      bool front = dot(q.n, d2) < 0.0f;
-      if ((in.flags & kInstMasked) && !faceAccepts(lp, in, front, q.u, q.v)) continue;
-      if (SHADOW) {
-        if (!(in.flags & kInstTransmissive)) return kTravOccluded;
-        uint16_t mid = front ? (uint16_t)(in.mats & 0xFFFF) : (uint16_t)(in.mats >> 16);
-        ShadePt spt = quadShade(in, q.n, q.u, q.v, sink.worldDir());
-        if (!shadowCross(lp, spt, mid, q.t, sink.worldDir(), trProd, tau)) return kTravOccluded;
-      } else {
-        t.tmax = q.t;
-        sink.hit(q.t, start, 0, q.u, q.v, q.n, front);
-      }
-    }
-    return binTravPop(t, stack, sink);
+  if (!t.inBlas) return binTravInstance<SHADOW, COUNT>(t, stack, lp, sink, trProd, tau, cnt);
+  while (true) {
+    const int r = binTravTriangle<SHADOW, COUNT>(t, stack, lp, sink, trProd, tau, cnt);
+    if (r != kTravLeaf) return r;
   }
-  // BLAS leaf: triangles in object space of curInst.
-  for (int k = 0; k < count; k++) {
-    const float4* tp = lp.tris + 3 * (size_t)(start + k);
-    float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
-    if (COUNT) cnt->triTests++;
-    float tt, b1, b2;
-    float3 p0 = v3(a.x, a.y, a.z), p1 = v3(b.x, b.y, b.z), p2 = v3(c.x, c.y, c.z);
-    if (!wtHit(t.wr, t.ro, p0, p1, p2, tmin, t.tmax, tt, b1, b2)) continue;
-    const int prim = __float_as_int(a.w);
-    const SdInstance& in = lp.inst[t.curInst];
-    if (!(in.flags & (kInstMasked | kInstTransmissive))) {
-      if (SHADOW) return kTravOccluded;
-      t.tmax = tt;
-      sink.hit(tt, t.curInst, prim, b1, b2, v3(0.0f), dot(cross(p1 - p0, p2 - p0), t.rd) < 0.0f);
-      continue;
-    }
-    ShadePt spt = triShade(lp, in, prim, b1, b2, sink.worldDir());
-    if ((in.flags & kInstMasked) && !faceAccepts(lp, in, spt.front, spt.u, spt.v)) continue;
-    if (SHADOW) {
-      if (!(in.flags & kInstTransmissive)) return kTravOccluded;
-      uint16_t mid = spt.front ? (uint16_t)(in.mats & 0xFFFF) : (uint16_t)(in.mats >> 16);
-      if (!shadowCross(lp, spt, mid, tt, sink.worldDir(), trProd, tau)) return kTravOccluded;
-    } else {
-      t.tmax = tt;
-      sink.hit(tt, t.curInst, prim, b1, b2, v3(0.0f), spt.front);
-    }
-  }
-  return binTravPop(t, stack, sink);
 }
 
 // Sink of a single traversal call: the world ray in registers, the closest

@@ -163,6 +163,16 @@ __global__ void __launch_bounds__(kRenderBlock) wfStart(unsigned long long base,
   }
 }
 
+// Lanes of each warp that take work from a list of n items: all of them when
+// the list fills the grid's lanes, else as few as spread it over every warp.
+// A short list is bound by the longest walk among the lanes that share a
+// warp, not by issue slots, so fewer lanes per warp end it sooner.
+__device__ __forceinline__ unsigned spreadLanes(unsigned n) {
+  const unsigned warps = gridDim.x * blockDim.x >> 5;
+  const unsigned per = max(1u, min(32u, (n + warps - 1) / warps));
+  return per == 32u ? 0xFFFFFFFFu : (1u << per) - 1u;
+}
+
 // Slot of ray i of the live list: the identity for the camera rays.
 template <bool CAM>
 __device__ __forceinline__ int liveSlot(int it, unsigned i) {
@@ -184,18 +194,28 @@ __device__ __forceinline__ void putMiss(float4* hits, int slot) {
   hits[2 * (size_t)slot] = make_float4(0.0f, __int_as_float(kMiss), 0.0f, 0.0f);
 }
 
-// Steps a lane may take in a row inside one round of the fetch loop, and
-// the fewest lanes still descending that keep the warp in the run (config 1
-// / config 0, Mrays/s; while any lane descends: 1 step 1,351 / 2,648; 4:
-// 1,459 / 2,697; 8: 1,497 / 2,723; 16: 1,512 / 2,726; 64: 1,499 / 2,709;
-// letting leaves continue the run too, 16 steps: 1,405 / 2,692; 16 steps
-// while at least 2 / 4 / 8 / 12 lanes descend: 1,555 / 2,713, 1,568 /
-// 2,718, 1,559 / 2,655, 1,525 / 2,680).
-#ifndef SDB_WF_INNER
-#define SDB_WF_INNER 16
+// A lane's next action.
+constexpr int kAtNode = 0, kAtTriangle = 1, kAtInstance = 2, kNoRay = 3;
+#if !SDB_WIDE_BVH
+__device__ __forceinline__ int travKind(const BinTrav& t) {
+  return t.cur >= 0 ? kAtNode : (t.inBlas ? kAtTriangle : kAtInstance);
+}
 #endif
-#ifndef SDB_WF_INNER_MIN
-#define SDB_WF_INNER_MIN 4
+// A round of the walk takes waiting instances if at least SDB_WF_INST_MIN
+// lanes have one (any, once the list is used up), then triangles one at a time
+// while at least SDB_WF_TRI_MIN lanes hold one, then node visits while at least
+// SDB_WF_NODE_MIN lanes are at one. Instancing 1080p, ms: every lane's own next
+// step, then descents (before) 96.0; 6 / 4 / 4 92.7; instances at 1 93.4; nodes
+// at 2 / 7 / 10 95.3 / 93.0 / 94.2; triangles at 1 / 8 95.1 / 94.4; always the
+// action most lanes wait for 98.6 (three small groups take turns).
+#ifndef SDB_WF_NODE_MIN
+#define SDB_WF_NODE_MIN 4
+#endif
+#ifndef SDB_WF_TRI_MIN
+#define SDB_WF_TRI_MIN 4
+#endif
+#ifndef SDB_WF_INST_MIN
+#define SDB_WF_INST_MIN 6
 #endif
 // Idle lanes a warp gathers before it fetches new rays (on the instancing
 // frame with the one-action loop: 894 Mrays/s at 24, 869 with a grid-stride
@@ -224,7 +244,7 @@ __device__ __forceinline__ void putMiss(float4* hits, int slot) {
 // group. The visit order and tests are those of traverse<false> in the
 // 8-wide build: the same closest accepted hit.
 template <bool SERVE, bool CAM>
-__global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetch(int it) {
+__global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetch(int it, bool) {
   const WfPool& pool = c_pool;
   const unsigned n = pool.counts[it].live;
   const unsigned full = 0xFFFFFFFFu;
@@ -405,11 +425,12 @@ struct PoolSink {
 constexpr float kRayMax = 1e16f;  // tmax of a radiance ray: any hit lowers it
 
 template <bool SERVE, bool CAM>
-__global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetch(int it) {
+__global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetch(int it, bool spread) {
   const WfPool& pool = c_pool;
   const unsigned n = pool.counts[it].live;
   const unsigned full = 0xFFFFFFFFu;
   const unsigned ltMask = (1u << (threadIdx.x & 31)) - 1u;
+  const unsigned lanes = spread ? spreadLanes(n) : full;
   int job = 0;  // SERVE: the lane's job slot
   int slot = -1;
   bool exhausted = false;  // warp-uniform
@@ -418,15 +439,15 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetc
   float trUnused = 1.0f;
   float3 tauUnused = v3(0.0f);
   while (true) {
-    const unsigned idle = __ballot_sync(full, slot < 0);
-    if (!exhausted && (idle == full || __popc(idle) >= SDB_WF_FETCH_IDLE)) {
+    const unsigned idle = __ballot_sync(full, slot < 0) & lanes;
+    if (!exhausted && (idle == lanes || __popc(idle) >= SDB_WF_FETCH_IDLE)) {
       const int leader = __ffs(idle) - 1;
       unsigned base = 0;
       if ((int)(threadIdx.x & 31) == leader)
         base = atomicAdd(&pool.counts[it].fetchRay, (unsigned)__popc(idle));
       base = __shfl_sync(full, base, leader);
       if (base + __popc(idle) >= n) exhausted = true;
-      if (slot < 0) {
+      if (idle >> (threadIdx.x & 31) & 1u) {
         unsigned i = base + __popc(idle & ltMask);
         if (i < n) {
           slot = liveSlot<CAM>(it, i);
@@ -443,19 +464,38 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetc
       if (exhausted) break;
       continue;
     }
-    // One step for every lane with a ray; then lanes that landed on an
-    // inner node keep descending (the while-while loop of Aila and Laine
-    // 2009 inside the dynamic-fetch loop) while at least SDB_WF_INNER_MIN of
-    // the warp's lanes do so, up to SDB_WF_INNER steps, before the warp
-    // meets again at the fetch vote; lanes at a leaf wait for the next round.
     const SdLaunch& lp = SERVE ? c_wjobs[job] : c_wlp;
     PoolSink sink{pool, slot};
     int r = kTravMore;
-    bool go = slot >= 0;
-    for (int k = 1;; k++) {
-      if (go) r = binTravStep<false, false>(t, stack, lp, sink, trUnused, tauUnused, nullptr);
-      go = slot >= 0 && r == kTravMore && t.cur >= 0;
-      if (k >= SDB_WF_INNER || __popc(__ballot_sync(full, go)) < SDB_WF_INNER_MIN) break;
+    // Leaves first (instances, then triangles one at a time while enough
+    // lanes hold one), then node visits in a row while enough lanes are at
+    // one; lanes that reach a leaf meanwhile wait for the next round.
+    int kind = slot < 0 ? kNoRay : travKind(t);
+    {
+      const int insts = __popc(__ballot_sync(full, kind == kAtInstance));
+      if (insts >= (exhausted ? 1 : SDB_WF_INST_MIN) || __ballot_sync(full, kind == kAtNode || kind == kAtTriangle) == 0) {
+        if (kind == kAtInstance) {
+          r = t.cur == kPop ? binTravPop(t, stack, sink)
+                            : binTravInstance<false, false>(t, stack, lp, sink, trUnused, tauUnused, nullptr);
+          kind = r == kTravMore ? travKind(t) : kNoRay;
+        }
+      }
+    }
+    for (int tris = __popc(__ballot_sync(full, kind == kAtTriangle)); tris > 0;) {
+      if (kind == kAtTriangle) {
+        r = binTravTriangle<false, false>(t, stack, lp, sink, trUnused, tauUnused, nullptr);
+        kind = r == kTravLeaf ? kAtTriangle : (r == kTravMore ? travKind(t) : kNoRay);
+      }
+      tris = __popc(__ballot_sync(full, kind == kAtTriangle));
+      if (tris < SDB_WF_TRI_MIN) break;
+    }
+    for (int nodes = __popc(__ballot_sync(full, kind == kAtNode)); nodes > 0;) {
+      if (kind == kAtNode) {
+        r = binTravNode<false, false>(t, stack, lp, sink, nullptr);
+        kind = r == kTravMore ? travKind(t) : kNoRay;
+      }
+      nodes = __popc(__ballot_sync(full, kind == kAtNode));
+      if (nodes < SDB_WF_NODE_MIN) break;
     }
     if (slot >= 0 && r == kTravDone) {
       if (t.tmax == kRayMax) putMiss(pool.hits, slot);
@@ -938,6 +978,7 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfShadowFet
   const unsigned n = pool.counts[it].shadow;
   const unsigned full = 0xFFFFFFFFu;
   const unsigned ltMask = (1u << (threadIdx.x & 31)) - 1u;
+  const unsigned lanes = spreadLanes(n);
   int slot = -1;
   bool exhausted = false;  // warp-uniform
   BinTrav t;
@@ -945,15 +986,15 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfShadowFet
   float trProd = 1.0f;
   float3 tau = v3(0.0f);
   while (true) {
-    const unsigned idle = __ballot_sync(full, slot < 0);
-    if (!exhausted && (idle == full || __popc(idle) >= SDB_WF_FETCH_IDLE)) {
+    const unsigned idle = __ballot_sync(full, slot < 0) & lanes;
+    if (!exhausted && (idle == lanes || __popc(idle) >= SDB_WF_FETCH_IDLE)) {
       const int leader = __ffs(idle) - 1;
       unsigned base = 0;
       if ((int)(threadIdx.x & 31) == leader)
         base = atomicAdd(&pool.counts[it].fetchShadow, (unsigned)__popc(idle));
       base = __shfl_sync(full, base, leader);
       if (base + __popc(idle) >= n) exhausted = true;
-      if (slot < 0) {
+      if (idle >> (threadIdx.x & 31) & 1u) {
         unsigned i = base + __popc(idle & ltMask);
         if (i < n) {
           slot = pool.shadowList[i];
@@ -972,13 +1013,37 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfShadowFet
     const SdLaunch& lp = slotLaunch<GUIDE>(slot >= 0 ? slot : 0);
     ShadowSink sink{pool, slot};
     int r = kTravMore;
-    bool go = slot >= 0;
-    for (int k = 1;; k++) {
-      if (go) r = binTravStep<true, false>(t, stack, lp, sink, trProd, tau, nullptr);
-      go = slot >= 0 && r == kTravMore && t.cur >= 0;
-      if (k >= SDB_WF_INNER || __popc(__ballot_sync(full, go)) < SDB_WF_INNER_MIN) break;
+    // Leaves first (instances, then triangles one at a time while enough
+    // lanes hold one), then node visits in a row while enough lanes are at
+    // one; lanes that reach a leaf meanwhile wait for the next round.
+    int kind = slot < 0 ? kNoRay : travKind(t);
+    {
+      const int insts = __popc(__ballot_sync(full, kind == kAtInstance));
+      if (insts >= (exhausted ? 1 : SDB_WF_INST_MIN) || __ballot_sync(full, kind == kAtNode || kind == kAtTriangle) == 0) {
+        if (kind == kAtInstance) {
+          r = t.cur == kPop ? binTravPop(t, stack, sink)
+                            : binTravInstance<true, false>(t, stack, lp, sink, trProd, tau, nullptr);
+          kind = r == kTravMore ? travKind(t) : kNoRay;
+        }
+      }
     }
-    if (slot >= 0 && r != kTravMore) {
+    for (int tris = __popc(__ballot_sync(full, kind == kAtTriangle)); tris > 0;) {
+      if (kind == kAtTriangle) {
+        r = binTravTriangle<true, false>(t, stack, lp, sink, trProd, tau, nullptr);
+        kind = r == kTravLeaf ? kAtTriangle : (r == kTravMore ? travKind(t) : kNoRay);
+      }
+      tris = __popc(__ballot_sync(full, kind == kAtTriangle));
+      if (tris < SDB_WF_TRI_MIN) break;
+    }
+    for (int nodes = __popc(__ballot_sync(full, kind == kAtNode)); nodes > 0;) {
+      if (kind == kAtNode) {
+        r = binTravNode<true, false>(t, stack, lp, sink, nullptr);
+        kind = r == kTravMore ? travKind(t) : kNoRay;
+      }
+      nodes = __popc(__ballot_sync(full, kind == kAtNode));
+      if (nodes < SDB_WF_NODE_MIN) break;
+    }
+    if (slot >= 0 && (r == kTravDone || r == kTravOccluded)) {
       float3 tr = v3(0.0f);
       if (r == kTravDone) {
         tau = v3(fmaxf(0.0f, tau.x), fmaxf(0.0f, tau.y), fmaxf(0.0f, tau.z));
@@ -1091,6 +1156,11 @@ void WfBuffers::ensure(int slots, bool withLate) {
   if (!counts.ptr) counts.alloc((kWfGroup + 1) * sizeof(WfCounts));
   pool.counts = (WfCounts*)counts.ptr;
   if (!hostCount) hostCount = pinnedWords();
+  if (!side) {
+    cudaCheck(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking), "shadow stream");
+    cudaCheck(cudaEventCreateWithFlags(&shaded, cudaEventDisableTiming), "shadow events");
+    cudaCheck(cudaEventCreateWithFlags(&shadowDone, cudaEventDisableTiming), "shadow events");
+  }
   cap = slots;
   late = withLate;
   gridTrace = gridFor(wfTraceFetch<false, false>);
@@ -1111,6 +1181,9 @@ WfBuffers::~WfBuffers() {
   if (hostCount) returnPinnedWords(hostCount);
   for (cudaEvent_t& e : ev)
     if (e) cudaEventDestroy(e);
+  if (shaded) cudaEventDestroy(shaded);
+  if (shadowDone) cudaEventDestroy(shadowDone);
+  if (side) cudaStreamDestroy(side);
 }
 
 // One idle pool per device, kept between sessions while the device-memory
@@ -1167,22 +1240,38 @@ template <int GUIDE, bool CAM>
 static int wfIteration(const WfBuffers& b, cudaStream_t st, int it, int depth,
                        unsigned long long base, const WfPlan& plan, bool timed) {
   int launches = 2;
+  // The shadow rays of an iteration and the radiance rays of the next need
+  // nothing of each other: without late vertices the shadow stage runs on the
+  // pool's second stream, beside the next trace, until the next shading.
+  const bool beside = plan.lights && !plan.late && !timed;
   if (timed) cudaEventRecord(b.ev[1], st);
-  wfTraceFetch<(GUIDE & kWfServe) != 0, CAM><<<b.gridTrace, kRenderBlock, 0, st>>>(it);
+  wfTraceFetch<(GUIDE & kWfServe) != 0, CAM><<<b.gridTrace, kRenderBlock, 0, st>>>(it, plan.shadowFetch);
   if (timed) cudaEventRecord(b.ev[2], st);
   if (plan.flames) {
     wfFlameScan<GUIDE, CAM><<<b.gridStart, kRenderBlock, 0, st>>>(it);
     wfFlame<GUIDE, CAM><<<b.gridFlame, kRenderBlock, 0, st>>>(it, depth, base);
     launches += 2;
   }
+  if (beside && !CAM) cudaCheck(cudaStreamWaitEvent(st, b.shadowDone, 0), "shadow stage");
   wfShade<GUIDE, CAM><<<b.gridShade, kShadeBlock, 0, st>>>(it, depth, base);
   if (timed) cudaEventRecord(b.ev[3], st);
   if (plan.lights) {
+    cudaStream_t ss = st;
+    if (beside) {
+      ss = b.side;
+      cudaCheck(cudaEventRecord(b.shaded, st), "shading stage");
+      cudaCheck(cudaStreamWaitEvent(ss, b.shaded, 0), "shading stage");
+    }
     if (plan.shadowFetch && !SDB_WIDE_BVH)
-      wfShadowFetch<GUIDE><<<b.gridShadow, kRenderBlock, 0, st>>>(it, depth);
+      wfShadowFetch<GUIDE><<<b.gridShadow, kRenderBlock, 0, ss>>>(it, depth);
     else
-      wfShadow<GUIDE><<<b.gridShadow, kRenderBlock, 0, st>>>(it, depth);
+      wfShadow<GUIDE><<<b.gridShadow, kRenderBlock, 0, ss>>>(it, depth);
     launches++;
+    if (beside) {
+      cudaCheck(cudaEventRecord(b.shadowDone, ss), "shadow stage");
+      if (depth + 1 >= plan.maxDepth || it + 1 == kWfGroup)  // back to one stream
+        cudaCheck(cudaStreamWaitEvent(st, b.shadowDone, 0), "shadow stage");
+    }
   }
   if (timed) cudaEventRecord(b.ev[4], st);
   if (plan.late) {

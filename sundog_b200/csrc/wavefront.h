@@ -62,6 +62,8 @@ struct WfBuffers {
   DevBuf trails;  // allocated by the first training-record pass
   unsigned* hostCount = nullptr;   // pinned: counters read back (from a process-wide free list)
   cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};  // stage timing
+  cudaStream_t side = nullptr;  // the shadow stage's, beside the next trace
+  cudaEvent_t shaded = nullptr, shadowDone = nullptr;
   int cap = 0;
   bool late = false;  // the slab holds late vertices
   int trailCap = 0;
