@@ -679,15 +679,17 @@ DevBvhStats buildBvhDevice(const float4* lo, const float4* hi, const float4* cen
   if (n <= maxLeaf) throw std::runtime_error("device BVH: a range this small is one leaf");
   if ((long long)primBase + n >= (1ll << 28)) throw std::runtime_error("device BVH: too many primitives");
   if (nodeCap < n - 1) throw std::runtime_error("device BVH: node array too small");
-  DevBuf ids0, ids1, ranges0, ranges1, counters;
-  ids0.alloc((size_t)n * sizeof(int));
-  ids1.alloc((size_t)n * sizeof(int));
-  ranges0.alloc((size_t)n * sizeof(BuildRange));
-  ranges1.alloc((size_t)n * sizeof(BuildRange));
-  counters.alloc(4 * sizeof(int));
-  cudaCheck(cudaMemsetAsync(counters.ptr, 0, counters.bytes, st), "device BVH counters");
-  int* cnt = (int*)counters.ptr;  // [0] nodes, [1] max depth, [2] next ranges, [3] error
-  bvhRoot<<<1, kBuildThreads, 0, st>>>(lo, hi, n, (int*)ids0.ptr, (BuildRange*)ranges0.ptr);
+  DevSlab slab;
+  const size_t aIds0 = slab.add((size_t)n * sizeof(int));
+  const size_t aIds1 = slab.add((size_t)n * sizeof(int));
+  const size_t aRanges0 = slab.add((size_t)n * sizeof(BuildRange));
+  const size_t aRanges1 = slab.add((size_t)n * sizeof(BuildRange));
+  const size_t aCounters = slab.add(4 * sizeof(int));
+  slab.alloc();
+  int* cnt = slab.at<int>(aCounters);
+  cudaCheck(cudaMemsetAsync(cnt, 0, 4 * sizeof(int), st), "device BVH counters");
+  // cnt: [0] nodes, [1] max depth, [2] next ranges, [3] error
+  bvhRoot<<<1, kBuildThreads, 0, st>>>(lo, hi, n, slab.at<int>(aIds0), slab.at<BuildRange>(aRanges0));
   cudaCheck(cudaGetLastError(), "device BVH root");
   BuildCtx c;
   c.lo = lo;
@@ -706,10 +708,10 @@ DevBvhStats buildBvhDevice(const float4* lo, const float4* hi, const float4* cen
   int* pinned = reinterpret_cast<int*>(pinnedWords());
   try {
     int nIn = 1;
-    void* idsIn = ids0.ptr;
-    void* idsOut = ids1.ptr;
-    void* rIn = ranges0.ptr;
-    void* rOut = ranges1.ptr;
+    void* idsIn = slab.at<void>(aIds0);
+    void* idsOut = slab.at<void>(aIds1);
+    void* rIn = slab.at<void>(aRanges0);
+    void* rOut = slab.at<void>(aRanges1);
     for (int level = 0; nIn > 0; level++) {
       if (level > 4096) throw std::runtime_error("device BVH: no progress");
       cudaCheck(cudaMemsetAsync(cnt + 2, 0, sizeof(int), st), "device BVH counters");
@@ -848,10 +850,11 @@ int collapseBvh4Device(const BvhNode* bin, int numBin, const int* roots, int num
                        Bvh4Node* out, int* outRoots, cudaStream_t st) {
   if (numRoots < 1 || numRoots > numBin)
     throw std::runtime_error("4-wide collapse: bad root count");
-  DevBuf items0, items1, counters;
-  items0.alloc((size_t)numBin * sizeof(Collapse4Item));
-  items1.alloc((size_t)numBin * sizeof(Collapse4Item));
-  counters.alloc(4 * sizeof(int));
+  DevSlab slab;
+  const size_t aItems0 = slab.add((size_t)numBin * sizeof(Collapse4Item));
+  const size_t aItems1 = slab.add((size_t)numBin * sizeof(Collapse4Item));
+  const size_t aCounters = slab.add(4 * sizeof(int));
+  slab.alloc();
   std::vector<Collapse4Item> first(numRoots);
   for (int r = 0; r < numRoots; r++) {
     if (roots[r] < 0 || roots[r] >= numBin)
@@ -859,10 +862,10 @@ int collapseBvh4Device(const BvhNode* bin, int numBin, const int* roots, int num
     first[r] = Collapse4Item{roots[r], r};
     outRoots[r] = r;
   }
-  cudaCheck(cudaMemcpyAsync(items0.ptr, first.data(), first.size() * sizeof(Collapse4Item),
+  cudaCheck(cudaMemcpyAsync(slab.at<void>(aItems0), first.data(), first.size() * sizeof(Collapse4Item),
                             cudaMemcpyHostToDevice, st),
             "4-wide collapse roots");
-  int* cnt = (int*)counters.ptr;  // [0] nodes, [1] next items, [2] error
+  int* cnt = slab.at<int>(aCounters);  // [0] nodes, [1] next items, [2] error
   int init[4] = {numRoots, 0, 0, 0};
   cudaCheck(cudaMemcpyAsync(cnt, init, sizeof init, cudaMemcpyHostToDevice, st),
             "4-wide collapse counters");
@@ -876,8 +879,8 @@ int collapseBvh4Device(const BvhNode* bin, int numBin, const int* roots, int num
   c.qCap = numBin;
   int host[4] = {0, 0, 0, 0};
   int nIn = numRoots;
-  void* in = items0.ptr;
-  void* nx = items1.ptr;
+  void* in = slab.at<void>(aItems0);
+  void* nx = slab.at<void>(aItems1);
   for (int level = 0; nIn > 0; level++) {
     if (level > 4096) throw std::runtime_error("4-wide collapse: no progress");
     cudaCheck(cudaMemsetAsync(cnt + 1, 0, sizeof(int), st), "4-wide collapse counters");

@@ -128,20 +128,17 @@ int flatGrid(int n) { return n <= 0 ? 1 : std::min((n + 255) / 256, 148 * 16); }
 DenoiseParams denoiseDefaults() { return DenoiseParams(); }
 
 void denoiseFilm(const float4* film, const float4* albedo, const float4* normal, int w, int h,
-                 const DenoiseParams& p, float4* out, cudaStream_t st) {
+                 const DenoiseParams& p, float4* work, float4* out, cudaStream_t st) {
   const int n = w * h;
   if (n <= 0) return;
   if (p.passes < 1 || p.passes > 8) throw std::runtime_error("denoise: passes must be 1..8");
-  DevBuf a, b;
-  a.alloc((size_t)n * sizeof(float4));
-  b.alloc((size_t)n * sizeof(float4));
-  demodulate<<<flatGrid(n), 256, 0, st>>>(film, albedo, n, (float4*)a.ptr);
+  float4* src = work;
+  float4* dst = work + n;
+  demodulate<<<flatGrid(n), 256, 0, st>>>(film, albedo, n, src);
   cudaCheck(cudaGetLastError(), "denoise demodulate");
   dim3 blk(16, 16), grd((w + 15) / 16, (h + 15) / 16);
-  spatialVariance<<<grd, blk, 0, st>>>((float4*)a.ptr, w, h);
+  spatialVariance<<<grd, blk, 0, st>>>(src, w, h);
   cudaCheck(cudaGetLastError(), "denoise variance");
-  float4* src = (float4*)a.ptr;
-  float4* dst = (float4*)b.ptr;
   for (int k = 0; k < p.passes; k++) {
     atrousPass<<<grd, blk, 0, st>>>(src, albedo, normal, w, h, 1 << k, p.sigmaLuminance,
                                     1.0f / (p.sigmaNormal * p.sigmaNormal),

@@ -1081,14 +1081,21 @@ using namespace sdb;
 
 namespace {
 
+// Device copy of a caller's network in a slab shared with the call's other
+// arrays.
 struct TmpNet {
-  DevBuf params, wbf;
-  explicit TmpNet(const float* p) {
-    params.alloc(kNetParams * sizeof(float));
-    cudaCheck(cudaMemcpy(params.ptr, p, kNetParams * sizeof(float), cudaMemcpyHostToDevice),
+  size_t aParams, aWbf;
+  const float* params = nullptr;
+  const bf16* wbf = nullptr;
+  explicit TmpNet(DevSlab& slab)
+      : aParams(slab.add(kNetParams * sizeof(float))), aWbf(slab.add(kNetWeights * sizeof(bf16))) {}
+  void load(const DevSlab& slab, const float* p) {
+    params = slab.at<float>(aParams);
+    wbf = slab.at<bf16>(aWbf);
+    cudaCheck(cudaMemcpy(slab.at<float>(aParams), p, kNetParams * sizeof(float),
+                         cudaMemcpyHostToDevice),
               "params");
-    wbf.alloc(kNetWeights * sizeof(bf16));
-    guideToBf16Kernel<<<(kNetWeights + 255) / 256, 256>>>((const float*)params.ptr, (bf16*)wbf.ptr);
+    guideToBf16Kernel<<<(kNetWeights + 255) / 256, 256>>>(params, slab.at<bf16>(aWbf));
     cudaCheck(cudaGetLastError(), "bf16");
   }
 };
@@ -1100,27 +1107,32 @@ extern "C" int sundog_guide_gradients(const float* params, const float* records,
   SDB_TRY
   if (!params || !records || !box || !grads || n <= 0) throw std::runtime_error("guide: bad arguments");
   enableSmem();
-  TmpNet net(params);
-  DevBuf rec, g, scal, cnt;
-  rec.upload(records, (size_t)n * kGuideRecordFloats * sizeof(float));
-  g.alloc(kNetParams * sizeof(float));
-  cudaCheck(cudaMemset(g.ptr, 0, g.bytes), "grads");
-  scal.alloc(2 * sizeof(float));
+  DevSlab slab;
+  TmpNet net(slab);
+  const size_t recBytes = (size_t)n * kGuideRecordFloats * sizeof(float);
+  const size_t aRec = slab.add(recBytes);
+  const size_t aGrads = slab.add(kNetParams * sizeof(float));
+  const size_t aScal = slab.add(2 * sizeof(float));
+  const size_t aCount = slab.add(sizeof(unsigned long long));
+  slab.alloc();
+  net.load(slab, params);
+  copyToDevice(slab.at<char>(aRec), records, recBytes);
+  cudaCheck(cudaMemset(slab.at<char>(aGrads), 0, kNetParams * sizeof(float)), "grads");
   double sum = 0.0;
   for (int i = 0; i < n; i++) sum += records[(size_t)i * kGuideRecordFloats + 3];
   float h[2] = {(float)sum, 0.0f};
-  cudaCheck(cudaMemcpy(scal.ptr, h, sizeof h, cudaMemcpyHostToDevice), "scalars");
+  cudaCheck(cudaMemcpy(slab.at<float>(aScal), h, sizeof h, cudaMemcpyHostToDevice), "scalars");
   unsigned long long cn = (unsigned long long)n;
-  cnt.upload(&cn, sizeof cn);
+  copyToDevice(slab.at<char>(aCount), &cn, sizeof cn);
   TrainArgs a;
-  a.wb = (const bf16*)net.wbf.ptr;
-  a.params = (const float*)net.params.ptr;
-  a.grads = (float*)g.ptr;
-  a.loss = (float*)scal.ptr + 1;
-  a.records = (const float4*)rec.ptr;
-  a.count = (const unsigned long long*)cnt.ptr;
+  a.wb = net.wbf;
+  a.params = net.params;
+  a.grads = slab.at<float>(aGrads);
+  a.loss = slab.at<float>(aScal) + 1;
+  a.records = slab.at<float4>(aRec);
+  a.count = slab.at<unsigned long long>(aCount);
   a.cap = cn;
-  a.sumF = (const float*)scal.ptr;
+  a.sumF = slab.at<float>(aScal);
   a.batch = n;
   a.sequential = 1;
   a.seed = 0;
@@ -1131,9 +1143,9 @@ extern "C" int sundog_guide_gradients(const float* params, const float* records,
   guideTrainKernel<<<std::min(tiles, smCount()), kThreads, kSmemTrain>>>(a);
   cudaCheck(cudaGetLastError(), "guide train");
   cudaCheck(cudaDeviceSynchronize(), "guide train");
-  cudaCheck(cudaMemcpy(grads, g.ptr, kNetParams * sizeof(float), cudaMemcpyDeviceToHost), "grads");
+  cudaCheck(cudaMemcpy(grads, slab.at<float>(aGrads), kNetParams * sizeof(float), cudaMemcpyDeviceToHost), "grads");
   if (loss) {
-    cudaCheck(cudaMemcpy(h, scal.ptr, sizeof h, cudaMemcpyDeviceToHost), "loss");
+    cudaCheck(cudaMemcpy(h, slab.at<float>(aScal), sizeof h, cudaMemcpyDeviceToHost), "loss");
     *loss = h[1];
   }
   return SUNDOG_OK;
@@ -1145,20 +1157,23 @@ extern "C" int sundog_guide_outputs(const float* params, const float* queries, i
   SDB_TRY
   if (!params || !queries || !outputs || n <= 0) throw std::runtime_error("guide: bad arguments");
   enableSmem();
-  TmpNet net(params);
-  DevBuf q, o;
-  q.upload(queries, (size_t)n * 6 * sizeof(float));
-  o.alloc((size_t)n * kNetLobeOut * sizeof(float));
+  DevSlab slab;
+  TmpNet net(slab);
+  const size_t qBytes = (size_t)n * 6 * sizeof(float), oBytes = (size_t)n * kNetLobeOut * sizeof(float);
+  const size_t aQueries = slab.add(qBytes), aOut = slab.add(oBytes);
+  slab.alloc();
+  net.load(slab, params);
+  copyToDevice(slab.at<char>(aQueries), queries, qBytes);
   ForwardArgs f;
-  f.wb = (const bf16*)net.wbf.ptr;
-  f.params = (const float*)net.params.ptr;
+  f.wb = net.wbf;
+  f.params = net.params;
   f.rows = n;
-  f.queries = (const float*)q.ptr;
-  f.outputs = (float*)o.ptr;
+  f.queries = slab.at<float>(aQueries);
+  f.outputs = slab.at<float>(aOut);
   f.lobes = nullptr;
   f.cdf = nullptr;
   runForwardTc(f, nullptr);
-  cudaCheck(cudaMemcpy(outputs, o.ptr, o.bytes, cudaMemcpyDeviceToHost), "outputs");
+  cudaCheck(cudaMemcpy(outputs, slab.at<float>(aOut), oBytes, cudaMemcpyDeviceToHost), "outputs");
   return SUNDOG_OK;
   SDB_CATCH(SUNDOG_ERROR)
 }

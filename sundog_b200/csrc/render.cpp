@@ -28,6 +28,7 @@
 #include "guide.h"
 #include "kernels.h"
 #include "cdf_build.h"
+#include "denoise.h"
 #include "render_session.h"
 #include "wavefront.h"
 #include "scene_model.h"
@@ -82,6 +83,10 @@ void DevBuf::upload(const void* src, size_t n) {
   alloc(n);
   if (n) cudaCheck(cudaMemcpy(ptr, src, n, cudaMemcpyHostToDevice), "upload");
   g_h2dBytes += n;
+}
+void copyToDevice(void* dst, const void* src, size_t bytes) {
+  if (bytes) cudaCheck(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice), "upload");
+  g_h2dBytes += bytes;
 }
 void DevBuf::release() {
   if (ptr) cudaFree(ptr);
@@ -441,12 +446,30 @@ void DeviceScene::build(const SceneDesc& desc) {
                        (Bvh4Node*)dNodes4.ptr, roots4.data(), 0);
     for (size_t i = 0; i < meshDescs.size(); i++) meshDescs[i].root = roots4[1 + i];
   }
-  dInst.upload(inst.data(), inst.size() * sizeof(SdInstance));
-  dMeshes.upload(meshDescs.data(), meshDescs.size() * sizeof(SdMesh));
-  dTex.upload(texDescs.data(), texDescs.size() * sizeof(SdTexture));
-  dMat.upload(scene.materials.data(), scene.materials.size() * sizeof(SdMaterial));
-  dLights.upload(lights.data(), lights.size() * sizeof(SdLight));
-  dFlames.upload(scene.flames.data(), scene.flames.size() * sizeof(SdFlame));
+  {
+    // The small arrays go up together: one allocation and one copy.
+    std::vector<char> staged;
+    std::vector<size_t> at;
+    auto stage = [&](const void* p, size_t bytes) {
+      at.push_back(staged.size());
+      staged.resize((staged.size() + bytes + 255) & ~(size_t)255);
+      if (bytes) std::memcpy(staged.data() + at.back(), p, bytes);
+    };
+    stage(inst.data(), inst.size() * sizeof(SdInstance));
+    stage(meshDescs.data(), meshDescs.size() * sizeof(SdMesh));
+    stage(texDescs.data(), texDescs.size() * sizeof(SdTexture));
+    stage(scene.materials.data(), scene.materials.size() * sizeof(SdMaterial));
+    stage(lights.data(), lights.size() * sizeof(SdLight));
+    stage(scene.flames.data(), scene.flames.size() * sizeof(SdFlame));
+    dArrays.upload(staged.data(), staged.size());
+    const char* base = (const char*)dArrays.ptr;
+    dInst = (const SdInstance*)(base + at[0]);
+    dMeshes = (const SdMesh*)(base + at[1]);
+    dTex = (const SdTexture*)(base + at[2]);
+    dMat = (const SdMaterial*)(base + at[3]);
+    dLights = (const SdLight*)(base + at[4]);
+    dFlames = (const SdFlame*)(base + at[5]);
+  }
   buildMs = msSince(tBuild);
   numLights = (int)lights.size();
   numObjects = nObj;
@@ -519,30 +542,36 @@ void DeviceScene::buildAccelOnDevice(const std::vector<HostMesh>& meshes,
       quadricBoundsHost(o.kind, d.qlo, d.qhi);
     }
   }
-  DevBuf dSrc, boxLo, boxHi, cent, order;
-  dSrc.upload(src.data(), src.size() * sizeof(DevInstanceSrc));
   size_t maxPrims = std::max<size_t>((size_t)nObj, 1);
   for (const HostMesh& m : meshes) maxPrims = std::max(maxPrims, m.idx.size());
-  boxLo.alloc(maxPrims * sizeof(float4));
-  boxHi.alloc(maxPrims * sizeof(float4));
-  cent.alloc(maxPrims * sizeof(float4));
-  order.alloc(maxPrims * sizeof(int));
-  instanceBoxesDevice((const DevInstanceSrc*)dSrc.ptr, nObj, (float4*)boxLo.ptr,
-                      (float4*)boxHi.ptr, (float4*)cent.ptr, st);
+  DevSlab scratch;
+  const size_t aSrc = scratch.add(src.size() * sizeof(DevInstanceSrc));
+  const size_t aLo = scratch.add(maxPrims * sizeof(float4));
+  const size_t aHi = scratch.add(maxPrims * sizeof(float4));
+  const size_t aCent = scratch.add(maxPrims * sizeof(float4));
+  const size_t aOrder = scratch.add(maxPrims * sizeof(int));
+  scratch.alloc();
+  copyToDevice(scratch.at<char>(aSrc), src.data(), src.size() * sizeof(DevInstanceSrc));
+  float4* const boxLo = scratch.at<float4>(aLo);
+  float4* const boxHi = scratch.at<float4>(aHi);
+  float4* const cent = scratch.at<float4>(aCent);
+  int* const order = scratch.at<int>(aOrder);
+  instanceBoxesDevice(scratch.at<DevInstanceSrc>(aSrc), nObj, boxLo,
+                      boxHi, cent, st);
   int cursor = 0;
   tlasOrder.assign(nObj, 0);
   if (nObj > 1) {
-    DevBvhStats t = buildBvhDevice((const float4*)boxLo.ptr, (const float4*)boxHi.ptr,
-                                   (const float4*)cent.ptr, nObj, 1, 0, 0, nodes, nObj - 1,
-                                   (int*)order.ptr, st);
-    cudaCheck(cudaMemcpy(tlasOrder.data(), order.ptr, nObj * sizeof(int), cudaMemcpyDeviceToHost),
+    DevBvhStats t = buildBvhDevice(boxLo, boxHi,
+                                   cent, nObj, 1, 0, 0, nodes, nObj - 1,
+                                   order, st);
+    cudaCheck(cudaMemcpy(tlasOrder.data(), order, nObj * sizeof(int), cudaMemcpyDeviceToHost),
               "TLAS order");
     tlasDepth = t.maxDepth;
     cursor = t.nodes;
   } else {
     float4 l, h;
-    cudaCheck(cudaMemcpy(&l, boxLo.ptr, sizeof l, cudaMemcpyDeviceToHost), "instance box");
-    cudaCheck(cudaMemcpy(&h, boxHi.ptr, sizeof h, cudaMemcpyDeviceToHost), "instance box");
+    cudaCheck(cudaMemcpy(&l, boxLo, sizeof l, cudaMemcpyDeviceToHost), "instance box");
+    cudaCheck(cudaMemcpy(&h, boxHi, sizeof h, cudaMemcpyDeviceToHost), "instance box");
     BvhNode root = singleLeafRoot({v3(l.x, l.y, l.z), v3(h.x, h.y, h.z)}, ~0);
     cudaCheck(cudaMemcpy(nodes, &root, sizeof root, cudaMemcpyHostToDevice), "TLAS root");
     tlasDepth = 0;
@@ -558,13 +587,13 @@ void DeviceScene::buildAccelOnDevice(const std::vector<HostMesh>& meshes,
     const int nt = (int)m.idx.size();
     meshDescs[i].root = cursor;
     if (nt > 4) {
-      meshBoxesDevice(meshDescs[i].pos, meshDescs[i].idx, nt, (float4*)boxLo.ptr,
-                      (float4*)boxHi.ptr, (float4*)cent.ptr, st);
-      DevBvhStats b = buildBvhDevice((const float4*)boxLo.ptr, (const float4*)boxHi.ptr,
-                                     (const float4*)cent.ptr, nt, 4, cursor, triCursor,
-                                     nodes + cursor, nt - 1, (int*)order.ptr, st);
+      meshBoxesDevice(meshDescs[i].pos, meshDescs[i].idx, nt, boxLo,
+                      boxHi, cent, st);
+      DevBvhStats b = buildBvhDevice(boxLo, boxHi,
+                                     cent, nt, 4, cursor, triCursor,
+                                     nodes + cursor, nt - 1, order, st);
       blasDepth = std::max(blasDepth, b.maxDepth);
-      gatherTrisDevice(meshDescs[i].pos, meshDescs[i].idx, (const int*)order.ptr, nt,
+      gatherTrisDevice(meshDescs[i].pos, meshDescs[i].idx, order, nt,
                        tris + 3 * (size_t)triCursor, st);
       cursor += b.nodes;
     } else {
@@ -582,9 +611,9 @@ void DeviceScene::buildAccelOnDevice(const std::vector<HostMesh>& meshes,
                             : singleLeafRoot({v3(3e30f), v3(3e30f)}, ~0);
       cudaCheck(cudaMemcpy(nodes + cursor, &root, sizeof root, cudaMemcpyHostToDevice), "BLAS root");
       if (nt > 0) {
-        cudaCheck(cudaMemcpy(order.ptr, ident.data(), nt * sizeof(int), cudaMemcpyHostToDevice),
+        cudaCheck(cudaMemcpy(order, ident.data(), nt * sizeof(int), cudaMemcpyHostToDevice),
                   "BLAS order");
-        gatherTrisDevice(meshDescs[i].pos, meshDescs[i].idx, (const int*)order.ptr, nt,
+        gatherTrisDevice(meshDescs[i].pos, meshDescs[i].idx, order, nt,
                          tris + 3 * (size_t)triCursor, st);
       }
       cursor += 1;
@@ -621,18 +650,18 @@ void DeviceScene::fillLaunch(SdLaunch& l) const {
   l.bgA = scene.bgA;
   l.bgB = scene.bgB;
   l.env = env;
-  l.textures = (const SdTexture*)dTex.ptr;
-  l.materials = (const SdMaterial*)dMat.ptr;
-  l.lights = (const SdLight*)dLights.ptr;
+  l.textures = dTex;
+  l.materials = dMat;
+  l.lights = dLights;
   l.numLights = numLights;
-  l.flames = (const SdFlame*)dFlames.ptr;
+  l.flames = dFlames;
   l.numFlames = (int)scene.flames.size();
   l.nodes = wideNodes ? nullptr : (const BvhNode*)dNodes.ptr;
   l.nodes4 = (const Bvh4Node*)dNodes4.ptr;
   l.cw = wideNodes ? (const CwNode*)dNodes.ptr : nullptr;
   l.tris = (const float4*)dTris.ptr;
-  l.inst = (const SdInstance*)dInst.ptr;
-  l.meshes = (const SdMesh*)dMeshes.ptr;
+  l.inst = dInst;
+  l.meshes = dMeshes;
   l.tlasRoot = 0;
   l.numInstances = numObjects;
 }
@@ -933,6 +962,15 @@ void RenderSession::countTraversal(sundog_trace_counts* out, sundog_trace_counts
     put(shadow, c[1], nullptr, c[1].traces);
     shadow->loop_iters = shadow->loop_lanes = 0;
   }
+}
+
+const float4* RenderSession::denoise() {
+  const size_t npix = (size_t)lp.width * lp.height;
+  if (!denoiseWork.ptr) denoiseWork.alloc(3 * npix * sizeof(float4));
+  float4* out = (float4*)denoiseWork.ptr;
+  denoiseFilm((const float4*)accum.ptr, (const float4*)aovAlb.ptr, (const float4*)aovNrm.ptr,
+              lp.width, lp.height, denoiseDefaults(), out + npix, out, stream);
+  return out;
 }
 
 void RenderSession::read(float* film, float* alb, float* nrm) {

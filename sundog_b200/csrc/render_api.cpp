@@ -187,13 +187,10 @@ int renderImpl(sundog_scene* h, const sundog_render_options* opt, const sundog_r
   // Optional post-process (src/capi_render.cpp:247-256): the denoised film
   // replaces the raw one as the call's output.
   double denoiseMs = 0.0;
-  DevBuf denoised;
+  const float4* denoised = nullptr;
   if (rs.denoise) {
     auto tDen = std::chrono::steady_clock::now();
-    denoised.alloc(npix * sizeof(float4));
-    denoiseFilm((const float4*)s->accum.ptr, (const float4*)s->aovAlb.ptr,
-                (const float4*)s->aovNrm.ptr, rs.width, rs.height, denoiseDefaults(),
-                (float4*)denoised.ptr, s->stream);
+    denoised = s->denoise();
     denoiseMs = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tDen).count();
   }
   // The film goes straight into the caller's buffer when there is one.
@@ -204,7 +201,7 @@ int renderImpl(sundog_scene* h, const sundog_render_options* opt, const sundog_r
     film = own.data();
   }
   if (rs.denoise) {
-    cudaCheck(cudaMemcpy(film, denoised.ptr, npix * sizeof(float4), cudaMemcpyDeviceToHost),
+    cudaCheck(cudaMemcpy(film, denoised, npix * sizeof(float4), cudaMemcpyDeviceToHost),
               "denoised film download");
     countDownload(npix * sizeof(float4));
   } else {
@@ -225,7 +222,7 @@ int renderImpl(sundog_scene* h, const sundog_render_options* opt, const sundog_r
     if (avif || endsWith(out, ".png")) {
       if (avif) out = out.substr(0, out.size() - 5) + ".png";
       std::vector<unsigned short> codes(npix * 3);
-      encodePq12((const float4*)(rs.denoise ? denoised.ptr : s->accum.ptr), rs.width, rs.height,
+      encodePq12((const float4*)(rs.denoise ? (const void*)denoised : s->accum.ptr), rs.width, rs.height,
                  rs.exposure, codes.data(), s->stream);
       writePq16Png(out, codes.data(), rs.width, rs.height);
       wrote = out;
@@ -262,11 +259,7 @@ extern "C" int sundog_session_denoise(sundog_session* sh, float* out) {
   RenderSession& s = *reinterpret_cast<RenderSession*>(sh);
   if (!s.aov) throw std::runtime_error("denoise: the session renders no AOVs (create it with AOVs)");
   size_t npix = (size_t)s.lp.width * s.lp.height;
-  DevBuf d;
-  d.alloc(npix * sizeof(float4));
-  denoiseFilm((const float4*)s.accum.ptr, (const float4*)s.aovAlb.ptr, (const float4*)s.aovNrm.ptr,
-              s.lp.width, s.lp.height, denoiseDefaults(), (float4*)d.ptr, s.stream);
-  cudaCheck(cudaMemcpy(out, d.ptr, npix * sizeof(float4), cudaMemcpyDeviceToHost), "denoise read");
+  cudaCheck(cudaMemcpy(out, s.denoise(), npix * sizeof(float4), cudaMemcpyDeviceToHost), "denoise read");
   countDownload(npix * sizeof(float4));
   return SUNDOG_OK;
   SDB_CATCH(SUNDOG_ERROR)

@@ -59,6 +59,26 @@ struct DevBuf {
   void release();
 };
 
+// Several arrays in one device allocation (an allocation and its free cost
+// more than most of the copies and kernels around them): add each array's
+// bytes, alloc() once, then take each one's address.
+struct DevSlab {
+  DevBuf buf;
+  size_t total = 0;
+  size_t add(size_t bytes) {
+    const size_t at = total;
+    total += (bytes + 255) & ~(size_t)255;
+    return at;
+  }
+  void alloc() { buf.alloc(total); }
+  template <typename T>
+  T* at(size_t offset) const {
+    return reinterpret_cast<T*>(static_cast<char*>(buf.ptr) + offset);
+  }
+};
+// Host-to-device copy into an existing buffer, counted as DevBuf::upload does.
+void copyToDevice(void* dst, const void* src, size_t bytes);
+
 struct MeshBufs {
   DevBuf pos, idx, nrm, uv;
 };
@@ -88,7 +108,14 @@ struct DeviceScene {
   std::vector<DevBuf> texImages;
   std::vector<MeshBufs> meshBufs;
   std::vector<DevBuf> lightBufs;
-  DevBuf dNodes, dTris, dInst, dMeshes, dTex, dMat, dLights, dFlames;
+  DevBuf dNodes, dTris;
+  DevBuf dArrays;  // instances, meshes, textures, materials, lights, flames
+  const SdInstance* dInst = nullptr;
+  const SdMesh* dMeshes = nullptr;
+  const SdTexture* dTex = nullptr;
+  const SdMaterial* dMat = nullptr;
+  const SdLight* dLights = nullptr;
+  const SdFlame* dFlames = nullptr;
   DevBuf dNodes4;  // the 4-wide layout (SDB_BVH4), collapsed from dNodes
   std::vector<SdLight> lights;  // host copy of the device light list
 
@@ -138,7 +165,12 @@ struct RenderSession {
   WfStageTimes stages;                // per-stage times of the last render
 
   ~RenderSession();
+  DevBuf denoiseWork;  // the denoised film and its scratch, from the first denoise on
+
   void build(const sundog_scene* h, const sundog_render_options* opt, const sundog_render_ext* ext);
+  // Denoises the film on the session's stream; the result stays in
+  // denoiseWork.
+  const float4* denoise();
   void render(cudaStream_t st, bool reset, sundog_render_result* res);
   void read(float* film, float* alb, float* nrm);
   // Counting render: traversal visit counts of both ray kinds in *out, or,

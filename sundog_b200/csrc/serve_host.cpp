@@ -41,26 +41,75 @@ static double msBetween(Clock::time_point a, Clock::time_point b) {
   return std::chrono::duration<double, std::milli>(b - a).count();
 }
 
-// Key of a scene's device data: its description without render settings and
-// camera (those are per film), plus the directory assets resolve against.
+// Key of a scene's device data: the bytes of its description without render
+// settings and camera (those are per film), plus the directory assets resolve
+// against. Fields of structs with pointers or padding go in one by one.
 static std::string sceneKey(const sundog_scene* h) {
-  size_t need = 0;
-  if (sundog_scene_debug_json(const_cast<sundog_scene*>(h), nullptr, 0, &need) != SUNDOG_OK)
-    throw std::runtime_error(sundog_last_error());
-  std::string js(need, '\0');
-  if (sundog_scene_debug_json(const_cast<sundog_scene*>(h), &js[0], need, &need) != SUNDOG_OK)
-    throw std::runtime_error(sundog_last_error());
-  size_t c = js.find("\"camera\":{");
-  if (c != std::string::npos) {
-    int depth = 0;
-    size_t i = js.find('{', c);
-    for (; i < js.size(); i++) {
-      if (js[i] == '{') depth++;
-      if (js[i] == '}' && --depth == 0) break;
-    }
-    js = js.substr(i + 1);
+  const SceneDesc& s = h->scene;
+  std::string k;
+  auto raw = [&](const void* p, size_t n) { k.append((const char*)p, n); };
+  auto num = [&](auto v) { raw(&v, sizeof v); };
+  auto text = [&](const std::string& t) {
+    num(t.size());
+    k += t;
+  };
+  text(s.baseDir);
+  num(s.bgKind);
+  num(s.bgA);
+  num(s.bgB);
+  text(s.env.file);
+  num(s.env.rotateDeg);
+  num(s.env.intensity);
+  num((int)s.env.importance);
+  num(s.textures.size());
+  for (const TextureCfg& t : s.textures) {
+    num(t.desc.kind);
+    num(t.desc.a);
+    num(t.desc.b);
+    num(t.desc.scale);
+    num(t.desc.width);
+    text(t.file);
+    num((int)t.srgb);
   }
-  return h->scene.baseDir + "\n" + js;
+  static_assert(sizeof(SdMaterial) == 14 * 4, "SdMaterial: 4-byte fields without padding");
+  num(s.materials.size());
+  raw(s.materials.data(), s.materials.size() * sizeof(SdMaterial));
+  num(s.meshes.size());
+  for (const MeshCfg& m : s.meshes) {
+    text(m.file);
+    text(m.usemtl);
+    num((int)m.smooth);
+  }
+  num(s.objects.size());
+  for (const ObjectCfg& o : s.objects) {
+    num(o.kind);
+    num(o.mesh);
+    num(o.matFront);
+    num(o.matBack);
+    num(o.cutoutTex);
+    num(o.xform);
+    num(o.lightId);
+    num((int)o.nee);
+  }
+  num(s.lights.size());
+  for (const SdLight& l : s.lights) {
+    num(l.kind);
+    num(l.p);
+    num(l.u);
+    num(l.v);
+    num(l.n);
+    num(l.L);
+    num(l.radius);
+    num(l.area);
+    num(l.dir);
+    num(l.twoSided);
+    num(l.texId);
+    num(l.flameId);
+  }
+  static_assert(sizeof(SdFlame) == 10 * 4, "SdFlame: 4-byte fields without padding");
+  num(s.flames.size());
+  raw(s.flames.data(), s.flames.size() * sizeof(SdFlame));
+  return k;
 }
 
 struct ServeJob {

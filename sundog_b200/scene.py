@@ -383,10 +383,10 @@ class Session(object):
 
     def read(self):
         s = self.stats
-        film = np.zeros((s.height, s.width, 4), np.float32)
+        film = np.empty((s.height, s.width, 4), np.float32)
         if self.aov:
-            alb = np.zeros_like(film)
-            nrm = np.zeros_like(film)
+            alb = np.empty_like(film)
+            nrm = np.empty_like(film)
             abi.check(self.lib.sundog_session_read(self.handle, film.ctypes.data, alb.ctypes.data,
                                                    nrm.ctypes.data), "read", self.lib)
             return film, alb, nrm
@@ -398,7 +398,7 @@ class Session(object):
         """The film denoised on the device (needs a session created with
         aov=True): height x width x 4 float32."""
         s = self.stats
-        out = np.zeros((s.height, s.width, 4), np.float32)
+        out = np.empty((s.height, s.width, 4), np.float32)
         abi.check(self.lib.sundog_session_denoise(self.handle, out.ctypes.data), "denoise",
                   self.lib)
         return out
