@@ -73,7 +73,7 @@ constexpr int kRound = (GUIDE & kWfServe) ? kRoundServe : kRoundStage;  // sd_bs
 #define SDB_WF_FLAME_BLOCKS 5
 #endif
 #ifndef SDB_WF_SHADE_BLOCKS
-#define SDB_WF_SHADE_BLOCKS 3
+#define SDB_WF_SHADE_BLOCKS 2
 #endif
 
 // A 32-byte record in one 256-bit load or store.
@@ -511,10 +511,10 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetc
 // needs (kClass*), so a warp runs one material's code instead of stepping
 // through all of them with a few lanes each.
 #ifndef SDB_SHADE_THREADS
-#define SDB_SHADE_THREADS 256
+#define SDB_SHADE_THREADS 384
 #endif
 #ifndef SDB_SHADE_TILE
-#define SDB_SHADE_TILE 1024
+#define SDB_SHADE_TILE 1536
 #endif
 constexpr int kShadeBlock = SDB_SHADE_THREADS;
 constexpr int kTileMax = SDB_SHADE_TILE;
@@ -802,6 +802,7 @@ __global__ void __launch_bounds__(kShadeBlock, SDB_WF_SHADE_BLOCKS) wfShade(
   __shared__ unsigned sList[3][kGroups];
   __shared__ unsigned sBase[3];
   __shared__ unsigned sPart[kWarps];
+  __shared__ unsigned sNext;
   const WfPool& pool = c_pool;
   WfCounts& cnt = pool.counts[it];
   const unsigned full = 0xFFFFFFFFu;
@@ -817,6 +818,7 @@ __global__ void __launch_bounds__(kShadeBlock, SDB_WF_SHADE_BLOCKS) wfShade(
   for (unsigned t0 = blockIdx.x * T; t0 < n; t0 += gridDim.x * T) {
     // Classes, and each entry's rank among its warp's entries of the class.
     for (int k = tid; k < kClasses * kGroups; k += kShadeBlock) sCount[k] = 0;
+    if (tid == 0) sNext = 0;
     __syncthreads();
     for (int k = 0; k < K; k++) {
       const int e = k * kShadeBlock + tid;
@@ -858,9 +860,17 @@ __global__ void __launch_bounds__(kShadeBlock, SDB_WF_SHADE_BLOCKS) wfShade(
       sOrder[sCount[(key >> 8) * kGroups + (e >> 5)] + (key & 0xFFu)] = (unsigned short)e;
     }
     __syncthreads();
-    for (int j = tid; j < shaded; j += kShadeBlock) {
-      const int e = sOrder[j];
-      sFlag[e] = (unsigned char)shadeRay<GUIDE, CAM>(pool, sSlot[e], base + t0 + e, depth);
+    // Warps take the sorted rays 32 at a time: classes cost unevenly.
+    while (true) {
+      unsigned j = 0;
+      if (lane == 0) j = atomicAdd(&sNext, 32u);
+      j = __shfl_sync(full, j, 0);
+      if (j >= (unsigned)shaded) break;
+      if (j + lane < (unsigned)shaded) {
+        const int e = sOrder[j + lane];
+        sFlag[e] = (unsigned char)shadeRay<GUIDE, CAM>(pool, sSlot[e], base + t0 + e, depth);
+      }
+      __syncwarp();
     }
     __syncthreads();
     // The tile's contributions to the next lists, in its own order.
@@ -877,10 +887,14 @@ __global__ void __launch_bounds__(kShadeBlock, SDB_WF_SHADE_BLOCKS) wfShade(
     }
     __syncthreads();
     if (warp < 3) {
+      // Two groups per lane.
+      static_assert(kGroups <= 64, "groups of a tile");
       unsigned total;
-      const bool in = lane < K * kWarps;
-      const unsigned ex = warpPrefix(in ? sList[warp][lane] : 0u, total);
-      if (in) sList[warp][lane] = ex;
+      const bool in0 = 2 * lane < K * kWarps, in1 = 2 * lane + 1 < K * kWarps;
+      const unsigned v0 = in0 ? sList[warp][2 * lane] : 0u, v1 = in1 ? sList[warp][2 * lane + 1] : 0u;
+      const unsigned ex = warpPrefix(v0 + v1, total);
+      if (in0) sList[warp][2 * lane] = ex;
+      if (in1) sList[warp][2 * lane + 1] = ex + v0;
       if (lane == 0 && total) {
         unsigned* c = warp == 0 ? &pool.counts[it + 1].live : (warp == 1 ? &cnt.shadow : &cnt.late);
         sBase[warp] = atomicAdd(c, total);
