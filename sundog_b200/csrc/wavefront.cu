@@ -152,8 +152,7 @@ __global__ void __launch_bounds__(kRenderBlock) wfStart(unsigned long long base,
     } else {
       ok = startPath(c_wlp, base + slot, p);
     }
-    if (!ok) {
-      pool.hits[2 * (size_t)slot] = make_float4(0.0f, __int_as_float(kNoPath), 0.0f, 0.0f);
+    if (!ok) {  // tile padding (isPadding)
       p.o = p.d = v3(0.0f);
       p.rng.state = 0;
     }
@@ -161,6 +160,13 @@ __global__ void __launch_bounds__(kRenderBlock) wfStart(unsigned long long base,
           make_float4(p.d.y, p.d.z, bitsF((unsigned)p.rng.state),
                       bitsF((unsigned)(p.rng.state >> 32))));
   }
+}
+
+// Whether a camera record is tile padding: no direction and no random state.
+// The state tells it from a camera ray whose direction vanished (a focus
+// distance whose square overflows), which is traced like any other.
+__device__ __forceinline__ bool isPadding(const Rec& r) {
+  return r.a.w == 0.0f && r.b.x == 0.0f && r.b.y == 0.0f && (bitsU(r.b.z) | bitsU(r.b.w)) == 0u;
 }
 
 // Lanes of each warp that take work from a list of n items: all of them when
@@ -192,6 +198,9 @@ __device__ __forceinline__ void putHit(float4* hits, int slot, float t, int inst
 }
 __device__ __forceinline__ void putMiss(float4* hits, int slot) {
   hits[2 * (size_t)slot] = make_float4(0.0f, __int_as_float(kMiss), 0.0f, 0.0f);
+}
+__device__ __forceinline__ void putNoPath(float4* hits, int slot) {
+  hits[2 * (size_t)slot] = make_float4(0.0f, __int_as_float(kNoPath), 0.0f, 0.0f);
 }
 
 // A lane's next action.
@@ -279,7 +288,10 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetc
           const Rec r = ldRec(pool.ray, slot);
           O = v3(r.a.x, r.a.y, r.a.z);
           D = v3(r.a.w, r.b.x, r.b.y);
-          if (CAM && D.x == 0.0f && D.y == 0.0f && D.z == 0.0f) slot = -1;  // tile padding
+          if (CAM && isPadding(r)) {
+            putNoPath(pool.hits, slot);
+            slot = -1;
+          }
           rayInit(ray, O, D, false);
           tmax = 1e16f;
           found = false;
@@ -456,7 +468,10 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetc
           const Rec r = ldRec(pool.ray, slot);
           const float3 o = v3(r.a.x, r.a.y, r.a.z), d = v3(r.a.w, r.b.x, r.b.y);
           binTravStart(t, jl, o, d, kRayMax);
-          if (CAM && d.x == 0.0f && d.y == 0.0f && d.z == 0.0f) slot = -1;  // tile padding
+          if (CAM && isPadding(r)) {
+            putNoPath(pool.hits, slot);
+            slot = -1;
+          }
         }
       }
     }

@@ -57,3 +57,20 @@ def test_deep_paths_match_megakernel(lib, depth):
     err = np.abs(a - b) / np.maximum(np.abs(b), 1e-3)
     assert np.quantile(err, 0.99) <= 1e-4
     assert abs(rays[0] - rays[1]) <= 2e-3 * rays[1]
+
+
+def test_vanished_camera_directions(lib):
+    """A focus distance whose square overflows leaves camera rays without a
+    direction. They are traced like any other (tile padding, which has no ray,
+    is not): here they meet nothing, so every pixel is the background."""
+    s = sc.Scene()
+    s.render(width=21, height=13, spp=3, max_depth=4, seed=2, clamp=0.0)
+    s.camera(lookfrom=[0, 0.3, 3.0], lookat=[0, 0, 0], vfov=40, focus_dist=1e20)
+    s.background_solid([0.25, 0.5, 0.75])
+    s.lambert("grey", color=[0.6, 0.6, 0.6])
+    s.add("sphere", "grey", sc.scale(0.15), sc.translate(0.3, 0.0, -0.4))
+    for engine in (0, 1):
+        with sc.Session(s, engine=engine) as ses:
+            assert ses.render().rays_traced == 21 * 13 * 3
+            assert np.array_equal(ses.read()[..., :3],
+                                  np.broadcast_to(np.float32([0.25, 0.5, 0.75]), (13, 21, 3)))
