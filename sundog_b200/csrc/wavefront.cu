@@ -1271,17 +1271,19 @@ static int wfIteration(const WfBuffers& b, cudaStream_t st, int it, int depth,
   int launches = 2;
   // The shadow rays of an iteration and the radiance rays of the next need
   // nothing of each other: without late vertices the shadow stage runs on the
-  // pool's second stream, beside the next trace, until the next shading.
+  // pool's second stream, beside the next trace, until the next flame march
+  // or shading.
   const bool beside = plan.lights && !plan.late && !timed;
   if (timed) cudaEventRecord(b.ev[1], st);
   wfTraceFetch<(GUIDE & kWfServe) != 0, CAM><<<b.gridTrace, kRenderBlock, 0, st>>>(it, plan.shadowFetch);
   if (timed) cudaEventRecord(b.ev[2], st);
+  // The flame march and shading read and write the radiance it adds to.
+  if (beside && !CAM) cudaCheck(cudaStreamWaitEvent(st, b.shadowDone, 0), "shadow stage");
   if (plan.flames) {
     wfFlameScan<GUIDE, CAM><<<b.gridStart, kRenderBlock, 0, st>>>(it);
     wfFlame<GUIDE, CAM><<<b.gridFlame, kRenderBlock, 0, st>>>(it, depth, base);
     launches += 2;
   }
-  if (beside && !CAM) cudaCheck(cudaStreamWaitEvent(st, b.shadowDone, 0), "shadow stage");
   wfShade<GUIDE, CAM><<<b.gridShade, kShadeBlock, 0, st>>>(it, depth, base);
   if (timed) cudaEventRecord(b.ev[3], st);
   if (plan.lights) {

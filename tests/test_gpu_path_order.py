@@ -9,7 +9,7 @@ launches: byte for byte."""
 import numpy as np
 import pytest
 
-from sundog_b200 import scene as sc
+from sundog_b200 import abi, scene as sc
 from sundog_b200 import workloads
 
 pytestmark = pytest.mark.gpu
@@ -74,3 +74,20 @@ def test_vanished_camera_directions(lib):
             assert ses.render().rays_traced == 21 * 13 * 3
             assert np.array_equal(ses.read()[..., :3],
                                   np.broadcast_to(np.float32([0.25, 0.5, 0.75]), (13, 21, 3)))
+
+
+def test_shadow_stage_beside_flames(lib, tmp_path):
+    """Opaque shadows in a scene with flames: shadow rays run on a second
+    stream beside the next trace, and the flame march after it reads the
+    radiance they add to. With stage timing everything runs on one stream:
+    the same film byte for byte."""
+    s = workloads.volumes(str(tmp_path), width=203, height=117, spp=5)
+    s.render(transparent_shadows=False)
+    with sc.Session(s, base_dir=str(tmp_path)) as ses:
+        abi.check(ses.lib.sundog_session_set_stage_timing(ses.handle, 1), "timing", ses.lib)
+        rays = ses.render().rays_traced
+        film = ses.read()
+        abi.check(ses.lib.sundog_session_set_stage_timing(ses.handle, 0), "timing", ses.lib)
+        for _ in range(3):
+            assert ses.render().rays_traced == rays
+            assert np.array_equal(ses.read(), film)
