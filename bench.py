@@ -310,8 +310,8 @@ def stage_roofline(lib, ses, stream, flush, rad, shd, peak, workload):
                      "bytes_per_ray": bpr, "achieved_gbps": ach,
                      "frac_of_hbm": ach / peak if ach else None,
                      "share_of_stage_time": ms / total if total else None}
-    for name, ms in (("wfStart", t.start_ms), ("wfShadeA", t.shade_a_ms),
-                     ("wfShadeB", t.shade_b_ms)):
+    for name, ms in (("wfStart", t.start_ms), ("wfShade", t.shade_a_ms),
+                     ("wfLate", t.shade_b_ms)):
         out[name] = {"ms_per_step": ms, "share_of_stage_time": ms / total if total else None}
     prof = profile_figures("wf_trace_l2_issue_%s.md" % workload) if workload else {}
     if prof:
@@ -338,6 +338,17 @@ def stage_roofline(lib, ses, stream, flush, rad, shd, peak, workload):
 
 
 # ---- CPU baseline (oracle on the host cores) ------------------------------------------
+
+def oracle_missing():
+    """Why the oracle cannot derive a scene here, or None: its scene code is
+    built from the reference's sources, which have to be mounted once."""
+    from oracle import oracle
+    try:
+        oracle.ref_scene_lib()
+    except RuntimeError as e:
+        return str(e)
+    return None
+
 
 def oracle_sample(scene, base_dir, args, seconds, threads):
     """Render a band of rows of the same frame with the CPU oracle."""
@@ -366,6 +377,10 @@ def oracle_sample(scene, base_dir, args, seconds, threads):
 def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return 0
+    why = oracle_missing()
+    if why:
+        print(json.dumps({"impl": "reference", "unavailable": why}), flush=True)
         return 0
     desc, published = resolve_workload(args)
     scene = make_scene(args)
@@ -605,7 +620,12 @@ def run_ours(args):
     if rank == 0:
         cpu = None
         if not args.no_cpu_baseline:
-            cpu, _, _ = oracle_sample(scene, base, args, args.cpu_seconds, os.cpu_count() or 1)
+            why = oracle_missing()
+            if why:
+                cpu = {"unavailable": why}
+            else:
+                cpu, _, _ = oracle_sample(scene, base, args, args.cpu_seconds,
+                                          os.cpu_count() or 1)
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world,
                 "steps": args.steps, "warmup": args.warmup,
                 "ms_per_step": total_ms / args.steps, "higher_is_better": True,
