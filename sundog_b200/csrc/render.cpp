@@ -807,7 +807,7 @@ void RenderSession::build(const sundog_scene* h, const sundog_render_options* op
   setupMs = msSince(tTotal);
 }
 
-// Wavefront pool size (slots, 285 B each; WfBuffers::ensure also caps it at
+// Wavefront pool size (slots, 193 B each; WfBuffers::ensure also caps it at
 // half the free device memory): up to 64 M, so a 32-spp chunk of a 1080p
 // frame (66 M paths) is almost all in flight at once and runs in about as
 // many iterations as its longest path has bounces. Measured on the instancing
