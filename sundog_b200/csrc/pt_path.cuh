@@ -28,13 +28,13 @@ __device__ __forceinline__ float3 background(const SdLaunch& lp, float3 dir) {
 }
 
 // Straight-line transmittance toward a light (device/programs.cu:70-85).
-template <bool COUNT>
+template <bool COUNT, bool LEAN = false>
 __device__ __forceinline__ float3 shadowTransmittance(const SdLaunch& lp, float3 o, float3 d,
                                                       float tmax, TraceCount* cnt) {
   TraceHit dummy;
   float trProd = 1.0f;
   float3 tau = v3(0.0f);
-  if (!traverse<true, COUNT>(lp, o, d, tmax, dummy, trProd, tau, cnt)) return v3(0.0f);
+  if (!traverse<true, COUNT, LEAN>(lp, o, d, tmax, dummy, trProd, tau, cnt)) return v3(0.0f);
   tau = v3(fmaxf(0.0f, tau.x), fmaxf(0.0f, tau.y), fmaxf(0.0f, tau.z));
   float3 tr = v3(trProd);
   if (hmax(tau) > 0.0f) tr = tr * vexp(-tau);
@@ -394,14 +394,17 @@ __device__ __forceinline__ bool bounce(const SdLaunch& lp, Path& p, unsigned lon
   TraceHit h;
   float dummyTr = 1.0f;
   float3 dummyTau = v3(0.0f);
-  const bool hit = traverse<false, COUNT>(lp, p.o, p.d, 1e16f, h, dummyTr, dummyTau, cnt);
+  // The megakernels are compiled for 32 registers.
+  constexpr bool kLean = ROUND == kRoundFree;
+  const bool hit = traverse<false, COUNT, kLean>(lp, p.o, p.d, 1e16f, h, dummyTr, dummyTau, cnt);
   rays++;
   Vertex v;
   crossMedia(lp, p, hit, h.t);
   if (!shadeSurface(lp, p, hit, h, rays, v)) return false;
   float3 tr = v3(0.0f);
   // Counting build: shadow traversals go to the second counter set.
-  if (v.nee) tr = shadowTransmittance<COUNT>(lp, v.so, v.wi, v.tmaxS, COUNT ? cnt + 1 : nullptr);
+  if (v.nee)
+    tr = shadowTransmittance<COUNT, kLean>(lp, v.so, v.wi, v.tmaxS, COUNT ? cnt + 1 : nullptr);
   return finishVertex<GUIDE, ROUND>(lp, p, v, tr, trail);
 }
 

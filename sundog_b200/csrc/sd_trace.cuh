@@ -382,7 +382,7 @@ constexpr uint32_t kGroupMarker = 1u << 30;  // entry returns from a BLAS
 // SHADOW = false: closest accepted hit, returns whether one was found.
 // SHADOW = true: returns false when occluded, else accumulates the
 // transparent-crossing terms into trProd / tau.
-template <bool SHADOW, bool COUNT = false>
+template <bool SHADOW, bool COUNT = false, bool LEAN = false>
 __device__ SDB_TRAVERSE_INLINE bool traverse(const SdLaunch& lp, float3 O, float3 D, float tmax,
                                              TraceHit& hit, float& trProd, float3& tau,
                                              TraceCount* cnt = nullptr) {
@@ -570,12 +570,13 @@ constexpr int kTravDone = 0;      // every node visited
 constexpr int kTravMore = 1;      // more steps to take
 constexpr int kTravOccluded = 2;  // shadow rays: an opaque crossing
 constexpr int kTravLeaf = 3;      // more triangles of the leaf to test
+constexpr int kTravPop = 4;       // nothing left to descend into: pop
 
-// Takes the next stack entry into t.cur, the step that ends a node or a leaf
-// with nothing left to descend into (done in that same step, so no loop
-// iteration is spent on a pop alone). A BLAS marker restores the world ray
-// and the entry below it is taken (a TLAS entry: BLASes do not nest).
-// Returns kTravDone when the stack is empty.
+// Takes the next stack entry into t.cur, the end of an action that left
+// nothing to descend into (in that same step, so no loop iteration is spent
+// on a pop alone). A BLAS marker restores the world ray and the entry below it
+// is taken (a TLAS entry: BLASes do not nest). Returns kTravDone when the stack
+// is empty.
 template <class Sink>
 __device__ __forceinline__ int binTravPop(BinTrav& t, TravStack& stack, Sink& sink) {
   if (t.sp == 0) return kTravDone;
@@ -592,8 +593,24 @@ __device__ __forceinline__ int binTravPop(BinTrav& t, TravStack& stack, Sink& si
   return kTravMore;
 }
 
+// The end of an action with nothing left to descend into: the pop itself
+// (POP: the stage kernels, whose rounds run one kind of action at a time), or
+// kTravPop for a caller with one pop for all actions.
+template <bool POP, class Sink>
+__device__ __forceinline__ int binTravEnd(BinTrav& t, TravStack& stack, Sink& sink) {
+  return POP ? binTravPop(t, stack, sink) : kTravPop;
+}
+
+// The actions of a walk. The sink receives what the walk finds and owns the
+// world ray: sink.world(ro, rd) restores it when the walk leaves a BLAS,
+// sink.worldDir() is the world direction for shading a candidate, and
+// (radiance rays) sink.hit(t, inst, prim, u, v, nq, front) takes each closer
+// accepted hit, t.tmax already lowered to it. Shadow rays multiply the
+// transparent crossings' Fresnel transmission into trProd and add their
+// signed optical depth into tau.
+
 // A TLAS leaf: one instance's quadric roots, or entry into its BLAS.
-template <bool SHADOW, bool COUNT, class Sink>
+template <bool SHADOW, bool COUNT, bool POP, class Sink>
 __device__ __forceinline__ int binTravInstance(BinTrav& t, TravStack& stack, const SdLaunch& lp,
                                                Sink& sink, float& trProd, float3& tau,
                                                TraceCount* cnt) {
@@ -605,19 +622,17 @@ __device__ __forceinline__ int binTravInstance(BinTrav& t, TravStack& stack, con
   if (in.kind == GK_MESH) {
     if (COUNT) cnt->blasEntries++;
     // Always room: the scene build bounds TLAS + BLAS depth by the stack.
-    if (t.sp < kStackSize) {
-      stack[t.sp++] = kToTlas;
-      t.inBlas = true;
-      t.curInst = start;
-      t.ro = o2;
-      t.rd = d2;
-      t.id = v3(safeInv(d2.x), safeInv(d2.y), safeInv(d2.z));
-      t.oi = o2 * t.id;
-      t.wr = wtSetup(d2);
-      t.cur = lp.meshes[in.mesh].root;
-      return kTravMore;
-    }
-    return binTravPop(t, stack, sink);
+    if (t.sp >= kStackSize) return binTravEnd<POP>(t, stack, sink);
+    stack[t.sp++] = kToTlas;
+    t.inBlas = true;
+    t.curInst = start;
+    t.ro = o2;
+    t.rd = d2;
+    t.id = v3(safeInv(d2.x), safeInv(d2.y), safeInv(d2.z));
+    t.oi = o2 * t.id;
+    t.wr = wtSetup(d2);
+    t.cur = lp.meshes[in.mesh].root;
+    return kTravMore;
   }
   if (COUNT) cnt->quadTests++;
   QHits qh = hitQuadric(in.kind, o2, d2, tmin, t.tmax);
@@ -636,52 +651,106 @@ __device__ __forceinline__ int binTravInstance(BinTrav& t, TravStack& stack, con
       sink.hit(q.t, start, 0, q.u, q.v, q.n, front);
     }
   }
-  return binTravPop(t, stack, sink);
+  return binTravEnd<POP>(t, stack, sink);
 }
 
-// One triangle of the current BLAS leaf, in object space of curInst. Returns
-// kTravLeaf while the leaf holds more (cur then names the rest), else pops.
+// Triangle `index` of the BLAS, in object space of curInst. False: occluded.
 template <bool SHADOW, bool COUNT, class Sink>
-__device__ __forceinline__ int binTravTriangle(BinTrav& t, TravStack& stack, const SdLaunch& lp,
-                                               Sink& sink, float& trProd, float3& tau,
-                                               TraceCount* cnt) {
-  const float tmin = 0.0f;
-  const int code = ~t.cur;
-  const float4* tp = lp.tris + 3 * (size_t)(code >> 3);
+__device__ __forceinline__ bool binTravTest(BinTrav& t, int index, const SdLaunch& lp, Sink& sink,
+                                            float& trProd, float3& tau, TraceCount* cnt) {
+  const float4* tp = lp.tris + 3 * (size_t)index;
   float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
   if (COUNT) cnt->triTests++;
   float tt, b1, b2;
   float3 p0 = v3(a.x, a.y, a.z), p1 = v3(b.x, b.y, b.z), p2 = v3(c.x, c.y, c.z);
-  if (wtHit(t.wr, t.ro, p0, p1, p2, tmin, t.tmax, tt, b1, b2)) {
-    const int prim = __float_as_int(a.w);
-    const SdInstance& in = lp.inst[t.curInst];
-    if (!(in.flags & (kInstMasked | kInstTransmissive))) {
-      if (SHADOW) return kTravOccluded;
-      t.tmax = tt;
-      sink.hit(tt, t.curInst, prim, b1, b2, v3(0.0f), dot(cross(p1 - p0, p2 - p0), t.rd) < 0.0f);
-    } else {
-      ShadePt spt = triShade(lp, in, prim, b1, b2, sink.worldDir());
-      if (!(in.flags & kInstMasked) || faceAccepts(lp, in, spt.front, spt.u, spt.v)) {
-        if (SHADOW) {
-          if (!(in.flags & kInstTransmissive)) return kTravOccluded;
-          uint16_t mid = spt.front ? (uint16_t)(in.mats & 0xFFFF) : (uint16_t)(in.mats >> 16);
-          if (!shadowCross(lp, spt, mid, tt, sink.worldDir(), trProd, tau)) return kTravOccluded;
-        } else {
-          t.tmax = tt;
-          sink.hit(tt, t.curInst, prim, b1, b2, v3(0.0f), spt.front);
-        }
-      }
-    }
+  if (!wtHit(t.wr, t.ro, p0, p1, p2, 0.0f, t.tmax, tt, b1, b2)) return true;
+  const int prim = __float_as_int(a.w);
+  const SdInstance& in = lp.inst[t.curInst];
+  if (!(in.flags & (kInstMasked | kInstTransmissive))) {
+    if (SHADOW) return false;
+    t.tmax = tt;
+    sink.hit(tt, t.curInst, prim, b1, b2, v3(0.0f), dot(cross(p1 - p0, p2 - p0), t.rd) < 0.0f);
+    return true;
   }
-  if (code & 7) {  // the next triangle of the leaf, one fewer left
-    t.cur = ~(code + 7);
-    return kTravLeaf;
+  ShadePt spt = triShade(lp, in, prim, b1, b2, sink.worldDir());
+  if ((in.flags & kInstMasked) && !faceAccepts(lp, in, spt.front, spt.u, spt.v)) return true;
+  if (SHADOW) {
+    if (!(in.flags & kInstTransmissive)) return false;
+    uint16_t mid = spt.front ? (uint16_t)(in.mats & 0xFFFF) : (uint16_t)(in.mats >> 16);
+    return shadowCross(lp, spt, mid, tt, sink.worldDir(), trProd, tau);
   }
-  return binTravPop(t, stack, sink);
+  t.tmax = tt;
+  sink.hit(tt, t.curInst, prim, b1, b2, v3(0.0f), spt.front);
+  return true;
+}
+
+// One triangle of the current BLAS leaf. Returns kTravLeaf while the leaf
+// holds more (cur then names the rest), else pops.
+template <bool SHADOW, bool COUNT, class Sink>
+__device__ __forceinline__ int binTravTriangle(BinTrav& t, TravStack& stack, const SdLaunch& lp,
+                                               Sink& sink, float& trProd, float3& tau,
+                                               TraceCount* cnt) {
+  const int code = ~t.cur;
+  if (!binTravTest<SHADOW, COUNT>(t, code >> 3, lp, sink, trProd, tau, cnt)) return kTravOccluded;
+  if (!(code & 7)) return binTravPop(t, stack, sink);
+  t.cur = ~(code + 7);  // the next triangle of the leaf, one fewer left
+  return kTravLeaf;
+}
+
+// The distance at which a ray enters a box, infinity when it misses it: the
+// larger of its near planes' distances against the smaller of its far ones'.
+__device__ __forceinline__ float boxEntry(float nx, float ny, float nz, float fx, float fy,
+                                          float fz, float tmin, float tmax) {
+  const float kFar = 1.00000024f;
+  const float n = fmaxf(fmaxf(nx, ny), fmaxf(nz, tmin));
+  const float f = fminf(fminf(fx, fy), fminf(fz, tmax)) * kFar;
+  return n <= f ? n : __int_as_float(0x7f800000);
+}
+
+// Entry distances of a 4-wide node's children: the near and far planes are
+// told by the ray's signs. LEAN takes two children at a time (half the planes
+// in registers at once) where the caller has few registers; otherwise all
+// four, as packed FMAs. The same distances bit for bit.
+template <bool LEAN>
+__device__ __forceinline__ void boxEntries(const float4* np, const BinTrav& t, float tmin, float& d0,
+                                           float& d1, float& d2, float& d3) {
+  const int sx = (int)(__float_as_uint(t.id.x) >> 31), sy = (int)(__float_as_uint(t.id.y) >> 31),
+            sz = (int)(__float_as_uint(t.id.z) >> 31);
+  if (LEAN) {
+    const float2* n2 = reinterpret_cast<const float2*>(np);
+    auto two = [&](int p, float& da, float& db) {
+      const float2 nx = __ldg(n2 + 2 * sx + p), fx = __ldg(n2 + 2 * (sx ^ 1) + p);
+      const float2 ny = __ldg(n2 + 4 + 2 * sy + p), fy = __ldg(n2 + 4 + 2 * (sy ^ 1) + p);
+      const float2 nz = __ldg(n2 + 8 + 2 * sz + p), fz = __ldg(n2 + 8 + 2 * (sz ^ 1) + p);
+      da = boxEntry(__fmaf_rn(nx.x, t.id.x, -t.oi.x), __fmaf_rn(ny.x, t.id.y, -t.oi.y),
+                    __fmaf_rn(nz.x, t.id.z, -t.oi.z), __fmaf_rn(fx.x, t.id.x, -t.oi.x),
+                    __fmaf_rn(fy.x, t.id.y, -t.oi.y), __fmaf_rn(fz.x, t.id.z, -t.oi.z), tmin, t.tmax);
+      db = boxEntry(__fmaf_rn(nx.y, t.id.x, -t.oi.x), __fmaf_rn(ny.y, t.id.y, -t.oi.y),
+                    __fmaf_rn(nz.y, t.id.z, -t.oi.z), __fmaf_rn(fx.y, t.id.x, -t.oi.x),
+                    __fmaf_rn(fy.y, t.id.y, -t.oi.y), __fmaf_rn(fz.y, t.id.z, -t.oi.z), tmin, t.tmax);
+    };
+    two(0, d0, d1);
+    two(1, d2, d3);
+    return;
+  }
+  const float4 nx = __ldg(np + sx), ny = __ldg(np + 2 + sy), nz = __ldg(np + 4 + sz);
+  const float4 fx = __ldg(np + (sx ^ 1)), fy = __ldg(np + 2 + (sy ^ 1)), fz = __ldg(np + 4 + (sz ^ 1));
+  const unsigned long long ix = pack2(t.id.x, t.id.x), iy = pack2(t.id.y, t.id.y), iz = pack2(t.id.z, t.id.z);
+  const unsigned long long mx = pack2(-t.oi.x, -t.oi.x), my = pack2(-t.oi.y, -t.oi.y), mz = pack2(-t.oi.z, -t.oi.z);
+  const float2 nx0 = fma2(pack2(nx.x, nx.y), ix, mx), nx1 = fma2(pack2(nx.z, nx.w), ix, mx);
+  const float2 ny0 = fma2(pack2(ny.x, ny.y), iy, my), ny1 = fma2(pack2(ny.z, ny.w), iy, my);
+  const float2 nz0 = fma2(pack2(nz.x, nz.y), iz, mz), nz1 = fma2(pack2(nz.z, nz.w), iz, mz);
+  const float2 fx0 = fma2(pack2(fx.x, fx.y), ix, mx), fx1 = fma2(pack2(fx.z, fx.w), ix, mx);
+  const float2 fy0 = fma2(pack2(fy.x, fy.y), iy, my), fy1 = fma2(pack2(fy.z, fy.w), iy, my);
+  const float2 fz0 = fma2(pack2(fz.x, fz.y), iz, mz), fz1 = fma2(pack2(fz.z, fz.w), iz, mz);
+  d0 = boxEntry(nx0.x, ny0.x, nz0.x, fx0.x, fy0.x, fz0.x, tmin, t.tmax);
+  d1 = boxEntry(nx0.y, ny0.y, nz0.y, fx0.y, fy0.y, fz0.y, tmin, t.tmax);
+  d2 = boxEntry(nx1.x, ny1.x, nz1.x, fx1.x, fy1.x, fz1.x, tmin, t.tmax);
+  d3 = boxEntry(nx1.y, ny1.y, nz1.y, fx1.y, fy1.y, fz1.y, tmin, t.tmax);
 }
 
 // A node visit: the boxes of its children.
-template <bool SHADOW, bool COUNT, class Sink>
+template <bool SHADOW, bool COUNT, bool LEAN, bool POP, class Sink>
 __device__ __forceinline__ int binTravNode(BinTrav& t, TravStack& stack, const SdLaunch& lp,
                                            Sink& sink, TraceCount* cnt) {
   const float tmin = 0.0f;
@@ -691,31 +760,9 @@ __device__ __forceinline__ int binTravNode(BinTrav& t, TravStack& stack, const S
   if (COUNT) cnt->boxTests += 4;
   const float inf = __int_as_float(0x7f800000);
   float d0, d1, d2, d3;
-  const int sx = (int)(__float_as_uint(t.id.x) >> 31), sy = (int)(__float_as_uint(t.id.y) >> 31),
-            sz = (int)(__float_as_uint(t.id.z) >> 31);
   const float4* np = reinterpret_cast<const float4*>(lp.nodes4 + t.cur);
-  const float4 nx = __ldg(np + sx), ny = __ldg(np + 2 + sy), nz = __ldg(np + 4 + sz);
-  const float4 fx = __ldg(np + (sx ^ 1)), fy = __ldg(np + 2 + (sy ^ 1)), fz = __ldg(np + 4 + (sz ^ 1));
   const int4 lk = __ldg(reinterpret_cast<const int4*>(np + 6));
-  const float kFar = 1.00000024f;
-  const unsigned long long ix = pack2(t.id.x, t.id.x), iy = pack2(t.id.y, t.id.y), iz = pack2(t.id.z, t.id.z);
-  const unsigned long long mx = pack2(-t.oi.x, -t.oi.x), my = pack2(-t.oi.y, -t.oi.y), mz = pack2(-t.oi.z, -t.oi.z);
-  const float2 nx0 = fma2(pack2(nx.x, nx.y), ix, mx), nx1 = fma2(pack2(nx.z, nx.w), ix, mx);
-  const float2 ny0 = fma2(pack2(ny.x, ny.y), iy, my), ny1 = fma2(pack2(ny.z, ny.w), iy, my);
-  const float2 nz0 = fma2(pack2(nz.x, nz.y), iz, mz), nz1 = fma2(pack2(nz.z, nz.w), iz, mz);
-  const float2 fx0 = fma2(pack2(fx.x, fx.y), ix, mx), fx1 = fma2(pack2(fx.z, fx.w), ix, mx);
-  const float2 fy0 = fma2(pack2(fy.x, fy.y), iy, my), fy1 = fma2(pack2(fy.z, fy.w), iy, my);
-  const float2 fz0 = fma2(pack2(fz.x, fz.y), iz, mz), fz1 = fma2(pack2(fz.z, fz.w), iz, mz);
-#define BOXT(D, NX, NY, NZ, FX, FY, FZ)                                               \
-  {                                                                                   \
-  const float n = fmaxf(fmaxf(NX, NY), fmaxf(NZ, tmin));                            \
-  const float f = fminf(fminf(FX, FY), fminf(FZ, t.tmax)) * kFar;                   \
-  D = n <= f ? n : inf;                                                             \
-  }
-  BOXT(d0, nx0.x, ny0.x, nz0.x, fx0.x, fy0.x, fz0.x)
-  BOXT(d1, nx0.y, ny0.y, nz0.y, fx0.y, fy0.y, fz0.y)
-  BOXT(d2, nx1.x, ny1.x, nz1.x, fx1.x, fy1.x, fz1.x)
-  BOXT(d3, nx1.y, ny1.y, nz1.y, fx1.y, fy1.y, fz1.y)
+  boxEntries<LEAN>(np, t, tmin, d0, d1, d2, d3);
   int l0 = lk.x, l1 = lk.y, l2 = lk.z, l3 = lk.w;
   // The nearest hit child first (three exchanges put the minimum in slot
   // 0); radiance rays also order the rest for front-to-back pops, shadow
@@ -728,7 +775,7 @@ __device__ __forceinline__ int binTravNode(BinTrav& t, TravStack& stack, const S
     cswap(d1, l1, d3, l3);
     cswap(d1, l1, d2, l2);
   }
-  if (!(d0 < inf)) return binTravPop(t, stack, sink);
+  if (!(d0 < inf)) return binTravEnd<POP>(t, stack, sink);
   // Always room: the scene build bounds the tree depths by the stack.
   if (d3 < inf && t.sp < kStackSize) stack[t.sp++] = l3;
   if (d2 < inf && t.sp < kStackSize) stack[t.sp++] = l2;
@@ -754,32 +801,42 @@ __device__ __forceinline__ int binTravNode(BinTrav& t, TravStack& stack, const S
   } else if (hb) {
     t.cur = nd.link.y;
   } else {
-    return binTravPop(t, stack, sink);
+    return binTravEnd<POP>(t, stack, sink);
   }
   return kTravMore;
 #endif
 }
 
-// One action of the walk. The sink receives what the walk finds and owns
-// the world ray: sink.world(ro, rd) restores it when the walk leaves a BLAS,
-// sink.worldDir() is the world direction for shading a candidate, and
-// (radiance rays) sink.hit(t, inst, prim, u, v, nq, front) takes each closer
-// accepted hit, t.tmax already lowered to it. Shadow rays multiply the
-// transparent crossings' Fresnel transmission into trProd and add their
-// signed optical depth into tau.
-template <bool SHADOW, bool COUNT, class Sink>
+// One action of the walk, and the pop that ends it where there is nothing to
+// descend into; all triangles of a leaf are one action. LEAN: boxEntries, and
+// one pop for all actions in place of one in each: the megakernels, at 32
+// registers, spill less (Cornell 512x512 at 16 spp 11.75 -> 10.42 ms,
+// instancing 960x540 23.0 -> 21.5, textured 7.9 -> 7.4; a megakernel server of
+// two scenes 16.0 -> 14.6).
+template <bool SHADOW, bool COUNT, bool LEAN, class Sink>
 __device__ __forceinline__ int binTravStep(BinTrav& t, TravStack& stack, const SdLaunch& lp,
                                            Sink& sink, float& trProd, float3& tau,
                                            TraceCount* cnt) {
   if (COUNT) countWarp(cnt, cnt->travIters, cnt->travLanes);
-  if (t.cur >= 0) return binTravNode<SHADOW, COUNT>(t, stack, lp, sink, cnt);
-  if (t.cur == kPop) return binTravPop(t, stack, sink);  // a walk with no TLAS
-  // Leaf: ~cur = start << 3 | (count - 1).
-  if (!t.inBlas) return binTravInstance<SHADOW, COUNT>(t, stack, lp, sink, trProd, tau, cnt);
-  while (true) {
-    const int r = binTravTriangle<SHADOW, COUNT>(t, stack, lp, sink, trProd, tau, cnt);
-    if (r != kTravLeaf) return r;
+  int r;
+  if (t.cur >= 0) {
+    r = binTravNode<SHADOW, COUNT, LEAN, !LEAN>(t, stack, lp, sink, cnt);
+  } else if (t.cur == kPop) {  // a walk with no TLAS
+    r = binTravEnd<!LEAN>(t, stack, sink);
+  } else if (!t.inBlas) {  // leaf: ~cur = start << 3 | (count - 1)
+    r = binTravInstance<SHADOW, COUNT, !LEAN>(t, stack, lp, sink, trProd, tau, cnt);
+  } else if (LEAN) {
+    const int start = ~t.cur >> 3, count = (~t.cur & 7) + 1;
+    for (int k = 0; k < count; k++)
+      if (!binTravTest<SHADOW, COUNT>(t, start + k, lp, sink, trProd, tau, cnt))
+        return kTravOccluded;
+    r = kTravPop;
+  } else {
+    do {
+      r = binTravTriangle<SHADOW, COUNT>(t, stack, lp, sink, trProd, tau, cnt);
+    } while (r == kTravLeaf);
   }
+  return LEAN && r == kTravPop ? binTravPop(t, stack, sink) : r;
 }
 
 // Sink of a single traversal call: the world ray in registers, the closest
@@ -808,8 +865,8 @@ struct RegisterSink {
 
 // SHADOW = false: closest accepted hit, returns whether one was found.
 // SHADOW = true: returns false when occluded, else accumulates the
-// transparent-crossing terms into trProd / tau.
-template <bool SHADOW, bool COUNT = false>
+// transparent-crossing terms into trProd / tau. LEAN: boxEntries.
+template <bool SHADOW, bool COUNT = false, bool LEAN = false>
 __device__ SDB_TRAVERSE_INLINE bool traverse(const SdLaunch& lp, float3 O, float3 D, float tmax,
                                              TraceHit& hit, float& trProd, float3& tau,
                                              TraceCount* cnt = nullptr) {
@@ -821,7 +878,7 @@ __device__ SDB_TRAVERSE_INLINE bool traverse(const SdLaunch& lp, float3 O, float
   RegisterSink sink{O, D, &hit, false};
   int r;
   do {
-    r = binTravStep<SHADOW, COUNT>(t, stack, lp, sink, trProd, tau, cnt);
+    r = binTravStep<SHADOW, COUNT, LEAN>(t, stack, lp, sink, trProd, tau, cnt);
   } while (r == kTravMore);
   if (SHADOW) return r == kTravDone;
   return sink.found;

@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetc
       if (insts >= (exhausted ? 1 : SDB_WF_INST_MIN) || __ballot_sync(full, kind == kAtNode || kind == kAtTriangle) == 0) {
         if (kind == kAtInstance) {
           r = t.cur == kPop ? binTravPop(t, stack, sink)
-                            : binTravInstance<false, false>(t, stack, lp, sink, trUnused, tauUnused, nullptr);
+                            : binTravInstance<false, false, true>(t, stack, lp, sink, trUnused, tauUnused, nullptr);
           kind = r == kTravMore ? travKind(t) : kNoRay;
         }
       }
@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfTraceFetc
     }
     for (int nodes = __popc(__ballot_sync(full, kind == kAtNode)); nodes > 0;) {
       if (kind == kAtNode) {
-        r = binTravNode<false, false>(t, stack, lp, sink, nullptr);
+        r = binTravNode<false, false, false, true>(t, stack, lp, sink, nullptr);
         kind = r == kTravMore ? travKind(t) : kNoRay;
       }
       nodes = __popc(__ballot_sync(full, kind == kAtNode));
@@ -1051,7 +1051,7 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfShadowFet
       if (insts >= (exhausted ? 1 : SDB_WF_INST_MIN) || __ballot_sync(full, kind == kAtNode || kind == kAtTriangle) == 0) {
         if (kind == kAtInstance) {
           r = t.cur == kPop ? binTravPop(t, stack, sink)
-                            : binTravInstance<true, false>(t, stack, lp, sink, trProd, tau, nullptr);
+                            : binTravInstance<true, false, true>(t, stack, lp, sink, trProd, tau, nullptr);
           kind = r == kTravMore ? travKind(t) : kNoRay;
         }
       }
@@ -1066,7 +1066,7 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfShadowFet
     }
     for (int nodes = __popc(__ballot_sync(full, kind == kAtNode)); nodes > 0;) {
       if (kind == kAtNode) {
-        r = binTravNode<true, false>(t, stack, lp, sink, nullptr);
+        r = binTravNode<true, false, false, true>(t, stack, lp, sink, nullptr);
         kind = r == kTravMore ? travKind(t) : kNoRay;
       }
       nodes = __popc(__ballot_sync(full, kind == kAtNode));
