@@ -29,7 +29,11 @@ CPP_SOURCES = ["scene_api.cpp", "scene_derive.cpp", "assets.cpp", "bvh_build.cpp
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ARCH + ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC",
                      "-Xcompiler", "-fvisibility=hidden", "--expt-relaxed-constexpr",
-                     "-Xptxas", "-warn-spills"]
+                     "-Xptxas", "-warn-spills",
+                     # nvcc compresses a unit's device code past some size; its
+                     # first launch then waits for the decompression (wavefront.cu:
+                     # the first render of a process 16 -> 8 ms without).
+                     "--no-compress"]
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-pthread", "-fvisibility=hidden", "-ffp-contract=off",
              "-Wall", "-Wno-unused-function", "-I" + os.path.join(CUDA_HOME, "include")]
 

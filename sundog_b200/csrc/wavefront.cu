@@ -1268,6 +1268,7 @@ struct WfPlan {
 template <int GUIDE, bool CAM>
 static int wfIteration(const WfBuffers& b, cudaStream_t st, int it, int depth,
                        unsigned long long base, const WfPlan& plan, bool timed) {
+  constexpr int kScene = GUIDE & kWfServe;  // stages that neither guide nor record
   int launches = 2;
   // The shadow rays of an iteration and the radiance rays of the next need
   // nothing of each other: without late vertices the shadow stage runs on the
@@ -1275,13 +1276,13 @@ static int wfIteration(const WfBuffers& b, cudaStream_t st, int it, int depth,
   // or shading.
   const bool beside = plan.lights && !plan.late && !timed;
   if (timed) cudaEventRecord(b.ev[1], st);
-  wfTraceFetch<(GUIDE & kWfServe) != 0, CAM><<<b.gridTrace, kRenderBlock, 0, st>>>(it, plan.shadowFetch);
+  wfTraceFetch<kScene != 0, CAM><<<b.gridTrace, kRenderBlock, 0, st>>>(it, plan.shadowFetch);
   if (timed) cudaEventRecord(b.ev[2], st);
   // The flame march and shading read and write the radiance it adds to.
   if (beside && !CAM) cudaCheck(cudaStreamWaitEvent(st, b.shadowDone, 0), "shadow stage");
   if (plan.flames) {
-    wfFlameScan<GUIDE, CAM><<<b.gridStart, kRenderBlock, 0, st>>>(it);
-    wfFlame<GUIDE, CAM><<<b.gridFlame, kRenderBlock, 0, st>>>(it, depth, base);
+    wfFlameScan<kScene, CAM><<<b.gridStart, kRenderBlock, 0, st>>>(it);
+    wfFlame<kScene, CAM><<<b.gridFlame, kRenderBlock, 0, st>>>(it, depth, base);
     launches += 2;
   }
   wfShade<GUIDE, CAM><<<b.gridShade, kShadeBlock, 0, st>>>(it, depth, base);
@@ -1294,9 +1295,9 @@ static int wfIteration(const WfBuffers& b, cudaStream_t st, int it, int depth,
       cudaCheck(cudaStreamWaitEvent(ss, b.shaded, 0), "shading stage");
     }
     if (plan.shadowFetch && !SDB_WIDE_BVH)
-      wfShadowFetch<GUIDE><<<b.gridShadow, kRenderBlock, 0, ss>>>(it, depth);
+      wfShadowFetch<kScene><<<b.gridShadow, kRenderBlock, 0, ss>>>(it, depth);
     else
-      wfShadow<GUIDE><<<b.gridShadow, kRenderBlock, 0, ss>>>(it, depth);
+      wfShadow<kScene><<<b.gridShadow, kRenderBlock, 0, ss>>>(it, depth);
     launches++;
     if (beside) {
       cudaCheck(cudaEventRecord(b.shadowDone, ss), "shadow stage");
