@@ -162,7 +162,8 @@ class Server {
     if (cfg.engine != 1) {  // the wavefront engine's slot pool, sized for a batch
       wf = wfAcquire();
       uint64_t batchPaths = cfg.iteration_paths + (uint64_t)kMaxServeJobs * maxItemPaths;
-      wf->ensure((int)std::min<uint64_t>(batchPaths, 1ull << 26), true);
+      batchSlots = (int)std::min<uint64_t>(batchPaths, 1ull << 26);
+      wf->ensure(batchSlots);
     }
     slots.assign(kMaxServeJobs, nullptr);
     thread = std::thread([this] { loop(); });
@@ -261,6 +262,7 @@ class Server {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   DevBuf scratch, dItems, counters;
   std::unique_ptr<WfBuffers> wf;  // engine 0: the wavefront engine's slot pool
+  int batchSlots = 0;             // the pool slots of a full batch
   ServeItem* hItems = nullptr;
   int maxItems = 0;
   uint64_t maxItemPaths = 0;
@@ -417,6 +419,12 @@ class Server {
       std::shared_ptr<DeviceScene> ds(new DeviceScene());
       ds->build(j->desc);
       it = sceneCache.emplace(j->key, CachedScene{ds, 0, 0}).first;
+      cudaCheck(cudaMemGetInfo(&freeB, &totB), "cudaMemGetInfo");
+    }
+    // Late vertices, from the first job on that may have some.
+    if (wf && wf->lateCap == 0 && !j->desc.flames.empty() &&
+        j->desc.render.transparentShadows) {
+      wf->ensureLate(batchSlots, filmBytes + cfg.reserve_bytes);
       cudaCheck(cudaMemGetInfo(&freeB, &totB), "cudaMemGetInfo");
     }
     if (freeB < filmBytes + cfg.reserve_bytes) {

@@ -129,6 +129,15 @@ __device__ __forceinline__ bool servePixel(unsigned long long id, int& job, int&
   return true;
 }
 
+// What a late vertex keeps beyond its path and its queued shadow ray (which
+// holds so, wi and tmaxS): the rest of Vertex.
+struct LateVertex {
+  float3 x, ns, albedo, Li;
+  float etaExt, etaRel, pdf, cosS;
+  int matId, lightK;
+  bool front, delta;
+};
+
 // Hit record markers (in place of the instance).
 constexpr int kMiss = -1;
 constexpr int kNoPath = -2;  // a slot of tile padding
@@ -690,7 +699,8 @@ __device__ __forceinline__ unsigned shadeRay(const WfPool& pool, int slot, unsig
           make_float4(v.wi.y, v.wi.z, v.tmaxS, bitsF(late ? kShadowLate : 0u)));
   if (late) {
     storePath(pool, p, slot);
-    pool.verts[slot].v = v;
+    pool.verts[slot].v = {v.x,   v.ns,   v.albedo, v.Li,    v.etaExt, v.etaRel,
+                          v.pdf, v.cosS, v.matId,  v.lightK, v.front,  v.delta};
     return 6;
   }
   int flags = (v.nee ? 1 : 0) | (v.delta ? 2 : 0) | (v.front ? 4 : 0);
@@ -1103,7 +1113,25 @@ __global__ void __launch_bounds__(kRenderBlock, SDB_WF_LATE_BLOCKS) wfLate(int i
     const SdLaunch& lp = slotLaunch<GUIDE>(slot);
     Path p;
     loadPath(pool, lp, slot, depth, p);
-    const Vertex v = pool.verts[slot].v;
+    const LateVertex l = pool.verts[slot].v;
+    const Rec r = ldRec(pool.shadowRays, slot);
+    Vertex v;
+    v.x = l.x;
+    v.ns = l.ns;
+    v.albedo = l.albedo;
+    v.etaExt = l.etaExt;
+    v.etaRel = l.etaRel;
+    v.matId = l.matId;
+    v.front = l.front;
+    v.nee = true;  // it waited for its shadow ray
+    v.lightK = l.lightK;
+    v.so = v3(r.a.x, r.a.y, r.a.z);
+    v.wi = v3(r.a.w, r.b.x, r.b.y);
+    v.Li = l.Li;
+    v.tmaxS = r.b.z;
+    v.pdf = l.pdf;
+    v.cosS = l.cosS;
+    v.delta = l.delta;
     const float4 tr = pool.shadowTerms[slot];
     GuideTrail* trail = (GUIDE & kGuideRecord) ? &pool.trails[slot].v : nullptr;
     if (finishVertex<GUIDE, kRound<GUIDE>>(lp, p, v, v3(tr.x, tr.y, tr.z), trail)) {
@@ -1143,30 +1171,26 @@ bool wfHasLate(const SdLaunch& lp, int guide) {
   return (guide & kGuideRecord) || (lp.numFlames > 0 && lp.transparentShadows);
 }
 
-void WfBuffers::ensure(int slots, bool withLate) {
-  if (slots <= cap && (late || !withLate)) return;
-  withLate = withLate || late;
-  slots = std::max(slots, cap);
+void WfBuffers::ensure(int slots) {
+  if (slots <= cap) return;
   // At most half of the device memory that is free (counting the pool about
   // to be replaced), so films, scenes and other work keep room; at least
   // 1 M slots.
   size_t freeB = 0, totB = 0;
   cudaCheck(cudaMemGetInfo(&freeB, &totB), "cudaMemGetInfo");
-  const size_t budget = (freeB + (size_t)cap * wfSlotBytes(late)) / 2;
-  const size_t fit = std::max<size_t>(budget / wfSlotBytes(withLate), (size_t)1 << 20);
+  const size_t budget = (freeB + (size_t)cap * wfSlotBytes()) / 2;
+  const size_t fit = std::max<size_t>(budget / wfSlotBytes(), (size_t)1 << 20);
   slots = (int)std::min<size_t>((size_t)slots, fit);
-  if (slots <= cap && late == withLate) return;
+  if (slots <= cap) return;
   const size_t n = (size_t)slots;
-  const size_t sizes[12] = {n * 32, n * 32, n * 32, n * 32, n * 32, n * 16,
-                            n * sizeof(int), n * sizeof(int), n * sizeof(int), n * sizeof(int), n,
-                            withLate ? n * sizeof(PoolSlot<Vertex>) : 0};
-  size_t offs[12], total = 0;
-  for (int k = 0; k < 12; k++) {
+  const size_t sizes[11] = {n * 32, n * 32, n * 32, n * 32, n * 32, n * 16,
+                            n * sizeof(int), n * sizeof(int), n * sizeof(int), n * sizeof(int), n};
+  size_t offs[11], total = 0;
+  for (int k = 0; k < 11; k++) {
     offs[k] = total;
     total += (sizes[k] + 255) & ~(size_t)255;
   }
   cap = 0;
-  late = false;
   slab.release();
   slab.alloc(total);
   char* base = (char*)slab.ptr;
@@ -1181,7 +1205,6 @@ void WfBuffers::ensure(int slots, bool withLate) {
   pool.shadowList = (int*)(base + offs[8]);
   pool.lateList = (int*)(base + offs[9]);
   pool.jobs = (unsigned char*)(base + offs[10]);
-  pool.verts = withLate ? (PoolSlot<Vertex>*)(base + offs[11]) : nullptr;
   if (!counts.ptr) counts.alloc((kWfGroup + 1) * sizeof(WfCounts));
   pool.counts = (WfCounts*)counts.ptr;
   if (!hostCount) hostCount = pinnedWords();
@@ -1191,13 +1214,30 @@ void WfBuffers::ensure(int slots, bool withLate) {
     cudaCheck(cudaEventCreateWithFlags(&shadowDone, cudaEventDisableTiming), "shadow events");
   }
   cap = slots;
-  late = withLate;
   gridTrace = gridFor(wfTraceFetch<false, false>);
   gridShade = gridFor(wfShade<0, false>, kShadeBlock);
   gridShadow = gridFor(wfShadow<0>);
   gridLate = gridFor(wfLate<0>);
   gridStart = gridFor(wfStart<0>);
   gridFlame = gridFor(wfFlame<0, false>);
+}
+
+void WfBuffers::ensureLate(int slots, size_t keep) {
+  slots = std::min(slots, cap);
+  if (slots <= lateCap) return;
+  // A buffer of its own, for the paths of the launches that have late
+  // vertices: a pool kept from a large frame is not made again for them.
+  // Half of the free memory at most, as the pool's.
+  size_t freeB = 0, totB = 0;
+  cudaCheck(cudaMemGetInfo(&freeB, &totB), "cudaMemGetInfo");
+  freeB += (size_t)lateCap * wfLateBytes();
+  const size_t fit = std::max<size_t>((freeB > keep ? freeB - keep : 0) / 2 / wfLateBytes(),
+                                      (size_t)1 << 20);
+  slots = (int)std::min<size_t>((size_t)slots, fit);
+  if (slots <= lateCap) return;
+  lateCap = 0;
+  verts.alloc((size_t)slots * wfLateBytes());
+  lateCap = slots;
 }
 
 void WfBuffers::ensureTrails() {
@@ -1249,9 +1289,8 @@ void wfReleaseIdle() {
   cudaSetDevice(cur);
 }
 
-size_t wfSlotBytes(bool withLate) {
-  return 6 * 32 - 16 + 4 * sizeof(int) + 1 + (withLate ? sizeof(PoolSlot<Vertex>) : 0);
-}
+size_t wfSlotBytes() { return 6 * 32 - 16 + 4 * sizeof(int) + 1; }
+size_t wfLateBytes() { return sizeof(PoolSlot<LateVertex>); }
 
 // What the launches of a render or batch need.
 struct WfPlan {
@@ -1339,11 +1378,15 @@ static int runPool(WfBuffers& b, cudaStream_t st, unsigned long long numPaths, c
     for (cudaEvent_t& e : b.ev) cudaCheck(cudaEventCreate(&e), "stage timing events");
   WfPool pool = b.pool;
   pool.trails = (PoolSlot<GuideTrail>*)b.trails.ptr;
+  pool.verts = (PoolSlot<LateVertex>*)b.verts.ptr;
+  // Paths in flight at once: slots, with a late vertex each where there can be some.
+  const int cap = plan.late ? std::min(b.cap, b.lateCap) : b.cap;
+  if (cap < 1) throw std::runtime_error("wavefront: no path slots");
   cudaCheck(cudaMemcpyToSymbolAsync(c_pool, &pool, sizeof pool, 0, cudaMemcpyHostToDevice, st),
             "wavefront pool");
   int launches = 0;
-  for (unsigned long long base = 0; base < numPaths; base += (unsigned long long)b.cap) {
-    const unsigned n = (unsigned)std::min<unsigned long long>((unsigned long long)b.cap,
+  for (unsigned long long base = 0; base < numPaths; base += (unsigned long long)cap) {
+    const unsigned n = (unsigned)std::min<unsigned long long>((unsigned long long)cap,
                                                               numPaths - base);
     cudaCheck(cudaMemsetAsync(b.counts.ptr, 0, b.counts.bytes, st), "wavefront counts");
     if (timed) cudaEventRecord(b.ev[0], st);

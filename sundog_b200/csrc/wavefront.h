@@ -10,7 +10,7 @@
 
 namespace sdb {
 
-struct Vertex;
+struct LateVertex;
 struct GuideTrail;
 
 // A pool entry at a 16-byte boundary, moved with 128-bit loads and stores.
@@ -44,7 +44,7 @@ struct WfPool {
   float4* hits;               // two: t, inst, prim | media << 30 | front << 31, u / v, normal.xyz
   float4* shadowRays;         // two: origin.xyz dir.xyz, tmax, flags
   float4* shadowTerms;        // the NEE term; for a late vertex its transmittance
-  PoolSlot<Vertex>* verts;    // late vertices (allocated when a launch may have some)
+  PoolSlot<LateVertex>* verts;  // late vertices, in a buffer of their own (WfBuffers::ensureLate)
   int* lists[2];              // live slot lists, ping-pong between iterations
   int *shadowList;
   int *lateList;              // late vertices; before shading, the rays that may meet a flame
@@ -60,12 +60,13 @@ struct WfBuffers {
   DevBuf slab, counts;
   WfPool pool = {};
   DevBuf trails;  // allocated by the first training-record pass
+  DevBuf verts;   // late vertices, from the first launch that may have some
   unsigned* hostCount = nullptr;   // pinned: counters read back (from a process-wide free list)
   cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};  // stage timing
   cudaStream_t side = nullptr;  // the shadow stage's, beside the next trace
   cudaEvent_t shaded = nullptr, shadowDone = nullptr;
   int cap = 0;
-  bool late = false;  // the slab holds late vertices
+  int lateCap = 0;   // slots with room for a late vertex
   int trailCap = 0;
   int gridStart = 0, gridTrace = 0, gridShade = 0, gridShadow = 0, gridLate = 0,
       gridFlame = 0;
@@ -73,9 +74,11 @@ struct WfBuffers {
   WfBuffers(const WfBuffers&) = delete;
   WfBuffers& operator=(const WfBuffers&) = delete;
   ~WfBuffers();
-  // Room for `slots` paths (fewer when device memory is short); withLate:
-  // with their late vertices.
-  void ensure(int slots, bool withLate);
+  // Room for `slots` paths (fewer when device memory is short).
+  void ensure(int slots);
+  // Room for the late vertices of `slots` of them (fewer when device memory
+  // is short; `keep` bytes of it are left free).
+  void ensureLate(int slots, size_t keep = 0);
   void ensureTrails();  // one GuideTrail per slot
 };
 
@@ -84,8 +87,9 @@ struct WfBuffers {
 // training record needs its radiance.
 bool wfHasLate(const SdLaunch& lp, int guide);
 
-// Device bytes per pool slot.
-size_t wfSlotBytes(bool withLate);
+// Device bytes per pool slot, and per late vertex.
+size_t wfSlotBytes();
+size_t wfLateBytes();
 // A pool for the current device: the idle one kept from an earlier session,
 // or a new empty one. wfRelease keeps a finished session's pool for reuse.
 std::unique_ptr<WfBuffers> wfAcquire();
