@@ -239,7 +239,9 @@ typedef struct sundog_session sundog_session;
 typedef struct {
   int32_t width, height, spp, chunk_spp;
   int32_t grid, block;           /* persistent launch shape */
-  uint64_t device_bytes;         /* device memory held by the session */
+  uint64_t device_bytes;         /* device memory held by the session (its
+                                    denoiser's buffers from the first denoise
+                                    on; not the path pool) */
   uint64_t bvh_nodes, triangles, instances;
   int32_t tlas_depth, blas_depth;
   double load_ms, build_ms, setup_ms;
@@ -295,8 +297,9 @@ SUNDOG_API int sundog_session_trace_counts_split(sundog_session*, sundog_trace_c
  * OptiX AI denoiser pass, src/denoise.cpp:18-53, with the same albedo and
  * normal guides): an edge-avoiding a-trous wavelet filter on the GPU. The
  * session must render AOVs (sundog_render_ext.aov_albedo or aov_normal set
- * at creation). out: width*height float4, host memory. sundog_render and
- * sundog_render_ex run the same filter when the scene or the options ask for
+ * at creation). out: width*height float4, host memory. The session keeps its
+ * buffers (48 bytes a pixel) for later calls; calls from several threads take
+ * turns. sundog_render and sundog_render_ex run the same filter when the scene or the options ask for
  * denoise, and write / return the denoised film. Returns 0/1. */
 SUNDOG_API int sundog_session_denoise(sundog_session*, float* out);
 

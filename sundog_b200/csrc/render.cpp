@@ -1072,14 +1072,17 @@ extern "C" int sundog_session_copy_film(sundog_session* sh, void* film_device, v
 extern "C" int sundog_session_info(sundog_session* sh, sundog_session_stats* st) {
   SDB_TRY
   if (!sh || !st) throw std::runtime_error("session: null argument");
-  const RenderSession* s = reinterpret_cast<RenderSession*>(sh);
+  RenderSession* s = reinterpret_cast<RenderSession*>(sh);
   st->width = s->lp.width;
   st->height = s->lp.height;
   st->spp = s->lp.sppTotal;
   st->chunk_spp = s->chunk;
   st->grid = s->grid;
   st->block = kRenderBlock;
-  st->device_bytes = s->deviceBytes;
+  {
+    std::lock_guard<std::mutex> lock(s->denoiseMu);
+    st->device_bytes = s->deviceBytes + s->denoiseWork.bytes;
+  }
   st->bvh_nodes = s->numNodes;
   st->triangles = s->numTris;
   st->instances = (uint64_t)s->lp.numInstances;

@@ -259,6 +259,7 @@ extern "C" int sundog_session_denoise(sundog_session* sh, float* out) {
   RenderSession& s = *reinterpret_cast<RenderSession*>(sh);
   if (!s.aov) throw std::runtime_error("denoise: the session renders no AOVs (create it with AOVs)");
   size_t npix = (size_t)s.lp.width * s.lp.height;
+  std::lock_guard<std::mutex> lock(s.denoiseMu);
   cudaCheck(cudaMemcpy(out, s.denoise(), npix * sizeof(float4), cudaMemcpyDeviceToHost), "denoise read");
   countDownload(npix * sizeof(float4));
   return SUNDOG_OK;

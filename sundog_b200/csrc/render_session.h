@@ -166,10 +166,12 @@ struct RenderSession {
 
   ~RenderSession();
   DevBuf denoiseWork;  // the denoised film and its scratch, from the first denoise on
+  std::mutex denoiseMu;
 
   void build(const sundog_scene* h, const sundog_render_options* opt, const sundog_render_ext* ext);
   // Denoises the film on the session's stream; the result stays in
-  // denoiseWork.
+  // denoiseWork. Callers that share the session with other threads hold
+  // denoiseMu until they have read it.
   const float4* denoise();
   void render(cudaStream_t st, bool reset, sundog_render_result* res);
   void read(float* film, float* alb, float* nrm);
