@@ -345,7 +345,7 @@ def oracle_missing():
     from oracle import oracle
     try:
         oracle.ref_scene_lib()
-    except RuntimeError as e:
+    except oracle.SceneCodeMissing as e:
         return str(e)
     return None
 

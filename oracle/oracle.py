@@ -8,8 +8,10 @@ into oracle/_ref/libsdref_scene.so by `make ref`), which derives the camera
 settings, transforms, NEE light registration and flame lights, and writes the
 result as the oracle's text description. The oracle loads that and renders
 pixel rectangles on the host cores. scene_text() turns a library's
-parse-time state (sundog_scene_debug_json) into the same description; the
-tests use it only to compare the product's derivation with the reference's.
+parse-time state (sundog_scene_debug_json) into the same description: the
+tests compare the product's derivation with the reference's through it, and
+where the reference's code was never built, renders are checked against the
+oracle's own integrator on the product's derivation.
 The module also exposes the oracle's function harness (sdo_fn) for
 per-function parity checks.
 
@@ -30,6 +32,11 @@ _lib = None
 _ref_scene = None
 
 
+class SceneCodeMissing(RuntimeError):
+    """sundog's own scene code was never built here (its sources were not
+    mounted)."""
+
+
 def build(force=False):
     """Compile the oracle with its Makefile, and the reference-built parts
     (function harness, scene library) when the reference sources are
@@ -48,17 +55,17 @@ def build(force=False):
 
 def ref_scene_lib():
     """sundog's own scene-construction library (oracle/_ref/libsdref_scene.so)
-    with the scene ABI's prototypes declared. Raises when it was never built:
-    it is built from the reference sources, which must be mounted once (the
-    built library then travels with the repository)."""
+    with the scene ABI's prototypes declared. Raises SceneCodeMissing when it
+    was never built: it is built from the reference sources, which must be
+    mounted once (the built library then travels with the repository)."""
     global _ref_scene
     if _ref_scene is None:
         if not os.path.isfile(REF_SCENE_LIB):
             build()
         if not os.path.isfile(REF_SCENE_LIB):
-            raise RuntimeError("oracle: %s is not built (it compiles sundog's own "
-                               "src/capi_scene.cpp and src/scene_build.cpp; mount the reference "
-                               "and run oracle.build())" % REF_SCENE_LIB)
+            raise SceneCodeMissing("oracle: %s is not built (it compiles sundog's own "
+                                   "src/capi_scene.cpp and src/scene_build.cpp; mount the "
+                                   "reference and run oracle.build())" % REF_SCENE_LIB)
         from sundog_b200 import abi
         lib = ctypes.CDLL(REF_SCENE_LIB, mode=ctypes.RTLD_LOCAL)
         abi.declare_scene_abi(lib)
