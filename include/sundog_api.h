@@ -203,8 +203,10 @@ typedef struct {
   int32_t engine;        /* path-tracing kernels: 0 = automatic (the
                             wavefront engine, guiding's training passes
                             included), 1 = persistent megakernel throughout,
-                            2 = same as 0. Both engines give the same
-                            samples. */
+                            2 = same as 0. Both engines take the same
+                            samples; their films agree to FP32 rounding
+                            (kernels compiled apart fuse other products), in
+                            which a path through glass or water may part. */
   int32_t shard_count;   /* > 1: render one tile shard of the frame, for one
                             GPU of shard_count: the 64x64 film tiles t
                             (row-major) with t % shard_count == shard_index.
@@ -285,14 +287,6 @@ SUNDOG_API int sundog_session_trace_counts(sundog_session*, sundog_trace_counts*
 SUNDOG_API int sundog_session_trace_counts_split(sundog_session*, sundog_trace_counts* radiance,
                                                  sundog_trace_counts* shadow);
 
-/* Per-stage device time of a session's wavefront renders (no counterpart in
- * the reference). With stage timing on, each later session_render records
- * CUDA events around every stage launch on its stream (read at the
- * synchronisation the engine makes once per iteration) and keeps, for the
- * last render: the summed milliseconds of the start, trace (radiance rays),
- * shade-A, shadow-ray and shade-B stages, the iterations, the radiance and
- * shadow rays traced and the stage launches. Megakernel renders leave it
- * zero. Returns 0/1. */
 /* Denoised copy of the session's film (the replacement of the reference's
  * OptiX AI denoiser pass, src/denoise.cpp:18-53, with the same albedo and
  * normal guides): an edge-avoiding a-trous wavelet filter on the GPU. The
@@ -340,6 +334,16 @@ SUNDOG_API int sundog_release_device_memory(void);
 SUNDOG_API int sundog_session_table(sundog_session*, int which, float* out, size_t cap,
                                     size_t* count);
 
+/* Per-stage device time of a session's wavefront renders (no counterpart in
+ * the reference). With stage timing on, each later session_render records
+ * CUDA events around every stage launch on its stream, reads them at a
+ * synchronisation per iteration (so such a render is slower) and keeps, for
+ * the last render: the summed milliseconds of the start stage (start_ms), the
+ * radiance rays' traversal (trace_ms), the flame scan and march with shading
+ * (shade_a_ms), the shadow rays (shadow_ms) and the late vertices, those that
+ * wait for their shadow ray (shade_b_ms); the iterations, the radiance and
+ * shadow rays traced and the stage launches. Megakernel renders leave it
+ * zero. Returns 0/1. */
 typedef struct {
   double start_ms, trace_ms, shade_a_ms, shadow_ms, shade_b_ms;
   uint64_t iterations, radiance_rays, shadow_rays, launches;
@@ -354,8 +358,9 @@ SUNDOG_API int sundog_session_stage_times(sundog_session*, sundog_stage_times*);
  * pixel rectangle (x0, y0, w, h) of a resident session's image and folds them
  * in sample order into film_device, w*h float4 running means in device memory
  * the caller owns (zeros for sample_begin 0). Sample indices count from the
- * session's first sample (its sample_offset), so the pixels equal the same
- * pixels of a full render of the session. Sessions with learned guiding
+ * session's first sample (its sample_offset), so these are the samples of the
+ * same pixels in a full render of the session (equal to it up to the FP32
+ * rounding of kernels compiled apart). Sessions with learned guiding
  * enabled are rejected (plain samples only). Calls no cudaMalloc/cudaFree:
  * its scratch is a static 16 MiB device array in the library (held by every
  * GPU that loads it until exit), so w*h*sample_count may not exceed 1048576

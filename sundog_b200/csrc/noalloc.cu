@@ -149,9 +149,10 @@ using namespace sdb;
 // sample order, into film_device: w*h float4 running means in the caller's
 // device memory (row-major, row 0 = image row y0), holding the means of the
 // samples before sample_begin (zeros when sample_begin is 0). Sample indices
-// count from the session's first sample (its sample_offset), as in a full
-// render of the session, so the result is identical to the same pixels of a
-// full render of it. Sessions with learned guiding enabled are rejected: this
+// count from the session's first sample (its sample_offset), so these are the
+// samples of the same pixels in a full render of the session (equal to it up
+// to the FP32 rounding of kernels compiled apart, Rounding in sd_bsdf.cuh).
+// Sessions with learned guiding enabled are rejected: this
 // entry point traces plain samples only. Allocates nothing. rays_out (host,
 // may be NULL) receives the radiance + shadow traces; when it is non-NULL
 // the call waits for the render to finish, otherwise the work is left queued

@@ -384,8 +384,8 @@ __device__ __forceinline__ bool finishVertex(const SdLaunch& lp, Path& p, const 
 // One segment of the path for the persistent kernels: the radiance ray,
 // crossMedia, shadeSurface, the shadow ray and finishVertex -- the functions the
 // wavefront stages call, in the same order with the same random draws, so
-// both engines trace the same samples. Returns false when the path has
-// ended. GUIDE selects the guided variants (kGuideSample: draw by MIS with
+// both engines trace the same samples up to FP32 rounding. Returns false when
+// the path has ended. GUIDE selects the guided variants (kGuideSample: draw by MIS with
 // the guide; kGuideRecord: keep training vertices in *trail); 0 is the
 // reference's sampler. (device/programs.cu:374-558)
 template <bool COUNT, int GUIDE = 0, int ROUND = kRoundFree>

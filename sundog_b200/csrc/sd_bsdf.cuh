@@ -15,9 +15,12 @@ namespace sdb {
 
 // Where the compiler may contract a product into a sum in more than one way,
 // what surrounds an inlined function decides, and a last bit that differs
-// sends a refracted path elsewhere. The kernels that must go on drawing the
-// samples they always drew name their form of the refraction instead:
-//   kRoundFree   left to the compiler (the persistent megakernel)
+// sends a refracted path elsewhere (volumes 320x180 at 8 spp: session, served
+// job, tile and megakernel films differ by up to 1.2% in 0.02% of the pixels,
+// by rounding in 5-8%; the same rays to 5 in 1.7 M). None of the forms is the
+// more exact one. They are named so that each way to render keeps its films
+// when the code around a refraction changes:
+//   kRoundFree   left to the compiler (the persistent megakernels)
 //   kRoundStage  the wavefront stages: smooth interfaces with a rounded
 //                cos^2, rough ones with a fused cos^2, and the order of every
 //                sum of products

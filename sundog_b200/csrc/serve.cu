@@ -11,8 +11,9 @@
 // constant-memory job table.
 //
 // ptServeFold folds each item's samples into its job's film in sample order
-// with the running mean of device/programs.cu:560-563, so a job's film is
-// bit-identical to a plain render of it.
+// with the running mean of device/programs.cu:560-563, so a job's film is the
+// same alone and in any mix, and a megakernel job's is bit-identical to a
+// megakernel session's.
 #include "pt_path.cuh"
 #include "serve.h"
 

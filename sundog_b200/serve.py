@@ -3,7 +3,7 @@ include/sundog_api.h): submit scenes as jobs, wait for their films.
 
     with Server(max_jobs=16) as sv:
         job = sv.submit(scene, width=512, height=512, spp=64)
-        film = job.wait()          # HxWx4 float32, bit-identical to a plain render
+        film = job.wait()          # HxWx4 float32, the same in any mix of jobs
 
 Several GPUs: MultiServer runs one server per device and places each job on
 the device with the least queued camera paths (jobs are independent, so a
