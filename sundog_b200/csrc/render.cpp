@@ -810,9 +810,10 @@ void RenderSession::build(const sundog_scene* h, const sundog_render_options* op
 // Wavefront pool size (slots, 193 B each; WfBuffers::ensure also caps it at
 // half the free device memory): up to 64 M, so a 32-spp chunk of a 1080p
 // frame (66 M paths) is almost all in flight at once and runs in about as
-// many iterations as its longest path has bounces. Measured on the instancing
-// frame: 894 / 981 / 1,049 / 1,092 / 1,115 Mrays/s at 4 / 8 / 16 / 32 / 64 M
-// slots (fewer iterations: fewer host round trips and stage-launch tails).
+// many iterations as its longest path has bounces. A smaller pool takes its
+// paths in turns, each through all its depths (the launches' tails): instancing
+// 1080p at 64 spp 199 / 118 / 95 / 89 ms at 1 / 4 / 16 / 64 M slots, volumes
+// 1440p at 32 spp 193 / 109 / 86 / 79.
 #ifndef SDB_WF_SLOTS_LOG2
 #define SDB_WF_SLOTS_LOG2 26
 #endif
