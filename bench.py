@@ -28,6 +28,7 @@ host cores, each step a bounded row sample of the same frame.
 
 import argparse
 import ctypes
+import hashlib
 import json
 import os
 import re
@@ -213,19 +214,48 @@ def measured_peaks():
     return 6650.0, "fallback"
 
 
+KERNEL_SOURCES = ("pt_kernel.cu", "wavefront.cu", "bvh_device.cu")
+
+
+def code_digest(csrc=os.path.join(ROOT, "sundog_b200", "csrc")):
+    """Digest of the path-tracing kernels' code: their sources and every
+    header, comments and spacing aside. A committed ncu summary names the
+    digest it was captured at."""
+    names = sorted(n for n in os.listdir(csrc) if n in KERNEL_SOURCES or n.endswith((".cuh", ".h")))
+    h = hashlib.sha256()
+    for n in names:
+        with open(os.path.join(csrc, n)) as f:
+            text = re.sub(r"//[^\n]*|/\*.*?\*/", " ", f.read(), flags=re.S)
+        h.update((n + " " + " ".join(text.split()) + "\n").encode())
+    return h.hexdigest()[:12]
+
+
+def profile_figures(name, folder=os.path.join(ROOT, "profiles"), code=None):
+    """`key: value` figures of a committed ncu summary (measured on a small
+    case), or {} when it is missing or its `code:` is not the present
+    kernels': counters of another kernel say nothing about this one's time."""
+    p = os.path.join(folder, name)
+    if not os.path.isfile(p):
+        return {}
+    with open(p) as f:
+        text = f.read()
+    m = re.search(r"^code:\s*(\w+)\s*$", text, re.M)
+    if not m or m.group(1) != (code or code_digest()):
+        return {}
+    return {m.group(1): float(m.group(2))
+            for m in re.finditer(r"^([a-z0-9_]+):\s*([0-9][0-9.eE+-]*)\s*$", text, re.M)
+            if m.group(1) != "code"}
+
+
 def ncu_traffic_per_path(engine=0):
     """DRAM bytes (read + write) per camera path of the path-tracing kernels,
     from the committed ncu summary of a smaller render of the same workload
     (traffic is per-path work: path state between stages, per-sample
     radiance writes, stack lines), so a chunk's traffic is this times its
-    paths. engine 1 = the persistent megakernel, else the wavefront engine."""
+    paths; None without a summary of the present kernels. engine 1 = the
+    persistent megakernel, else the wavefront engine."""
     name = "pt_persistent_instancing.md" if engine == 1 else "wf_render_dram_instancing_small.md"
-    p = os.path.join(ROOT, "profiles", name)
-    if not os.path.isfile(p):
-        return None
-    with open(p) as f:
-        m = re.search(r"dram_bytes_per_path:\s*([0-9.eE+]+)", f.read())
-    return float(m.group(1)) if m else None
+    return profile_figures(name).get("dram_bytes_per_path")
 
 
 # Algorithmic bytes of the traversal on the BVH it walks (the library's 4-wide
@@ -243,18 +273,6 @@ def sum_counts(a, b):
     for f, _ in abi.TraceCounts._fields_:
         setattr(c, f, getattr(a, f) + (0 if f.startswith("loop") else getattr(b, f)))
     return c
-
-
-def profile_figures(name):
-    """`key: value` figures of a committed ncu summary under profiles/ (the
-    measured L2 bytes and issue-slot use of a kernel on a small case)."""
-    p = os.path.join(ROOT, "profiles", name)
-    out = {}
-    if os.path.isfile(p):
-        with open(p) as f:
-            for m in re.finditer(r"^([a-z0-9_]+):\s*([0-9.eE+-]+)\s*$", f.read(), re.M):
-                out[m.group(1)] = float(m.group(2))
-    return out
 
 
 def l2_copy_gbps(stream):
@@ -289,7 +307,8 @@ def stage_roofline(lib, ses, stream, flush, rad, shd, peak, workload):
     `value`) with per-stage CUDA events: each stage kernel's own time, and for
     the two traversal stages their algorithmic bytes (radiance and shadow
     rays counted apart) over that time. L2 bytes and issue-slot utilisation
-    come from the committed small-case ncu summary of the trace stage."""
+    come from the committed small-case ncu summary of the trace stage, if it is
+    of the present kernels."""
     import torch
     from sundog_b200 import abi
     abi.check(lib.sundog_session_set_stage_timing(ses.handle, 1), "stage timing", lib)
@@ -310,7 +329,8 @@ def stage_roofline(lib, ses, stream, flush, rad, shd, peak, workload):
                      "bytes_per_ray": bpr, "achieved_gbps": ach,
                      "frac_of_hbm": ach / peak if ach else None,
                      "share_of_stage_time": ms / total if total else None}
-    for name, ms in (("wfStart", t.start_ms), ("wfShade", t.shade_a_ms),
+    # The second is one interval: scenes with flames run all three in it.
+    for name, ms in (("wfStart", t.start_ms), ("wfFlameScan + wfFlame + wfShade", t.shade_a_ms),
                      ("wfLate", t.shade_b_ms)):
         out[name] = {"ms_per_step": ms, "share_of_stage_time": ms / total if total else None}
     prof = profile_figures("wf_trace_l2_issue_%s.md" % workload) if workload else {}
