@@ -200,14 +200,20 @@ extern "C" int sundog_session_render_tile_noalloc(sundog_session* sh, int x0, in
   cudaCheck(cudaGetLastError(), "noalloc set-up launch");
   long long total = (long long)w * h * sample_count;
   // A small tile is bound by its longest warp, so its paths are spread over
-  // more warps than they fill: over 16 per SM where walks or flame marches are
-  // long (volumes 18x18 at 6 samples 157 -> 113 us, instancing 40x40 at 9
-  // 362 -> 311; at 2 per SM 128 and 376), over one per SM where they are short
-  // (Cornell 8x8 at 1 sample 92 -> 58 us; 32x32 at 4 takes 111 us in full
-  // warps, 117 over 2 per SM and 120 over 16: paths in step share their
-  // instruction fetches).
+  // more warps than they fill: one per SM where walks are short (Cornell 8x8 at
+  // 1 sample 92 -> 58 us; 32x32 at 4 takes 111 us in full warps, 117 over 2 per
+  // SM and 120 over 16: paths in step share their instruction fetches). Where
+  // walks or flame marches are long, 16 per SM while that gives a warp up to
+  // two paths (volumes 18x18 at 6 samples 157 -> 113 us, instancing 40x40 at 9
+  // 362 -> 311), 5 per SM beyond: volumes 64x64 at 4 samples takes 382 us over
+  // 16 and 273 over 5, 40x40 at 16 398 and 279, instancing 24x24 at 64 536 and
+  // 486; at 4,096 paths neither leads (volumes 32x32 at 4 187 over 16 and 166
+  // over 5, instancing 207 and 237).
+  int dev = 0, sms = 0;
+  cudaCheck(cudaGetDevice(&dev), "cudaGetDevice");
+  cudaCheck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
   const bool uneven = lp.numInstances >= kShadowFetchInstances || lp.numFlames > 0;
-  const long long spread = 148 * (uneven ? 16 : 1);
+  const long long spread = (long long)sms * (!uneven ? 1 : total <= 32ll * sms ? 16 : 5);
   const int lanes = (int)std::min<long long>(32, (total + spread - 1) / spread);
   const long long warps = (total + lanes - 1) / lanes;
   int grid = (int)((warps * 32 + kRenderBlock - 1) / kRenderBlock);
