@@ -20,7 +20,9 @@ void countDownload(size_t bytes);
 
 // Per-stage device time of wavefront renders, accumulated while a session
 // has stage timing on: CUDA events on the render stream around each stage
-// launch, read at the per-iteration synchronisation the engine makes anyway.
+// launch, read at a synchronisation made per iteration for them (which also
+// keeps the shadow stage on the one stream). shadeAMs is the flame scan, the
+// flame march and shading, shadeBMs the late vertices.
 struct WfStageTimes {
   double startMs = 0, traceMs = 0, shadeAMs = 0, shadowMs = 0, shadeBMs = 0;
   unsigned long long iterations = 0, radianceRays = 0, shadowRays = 0, launches = 0;

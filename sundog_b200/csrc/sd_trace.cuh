@@ -767,7 +767,7 @@ __device__ __forceinline__ int binTravNode(BinTrav& t, TravStack& stack, const S
   // The nearest hit child first (three exchanges put the minimum in slot
   // 0); radiance rays also order the rest for front-to-back pops, shadow
   // rays, which stop at any opaque hit, take them as found (shadow stage
-  // 119.0 -> 115.6 ms on config 2, 22.9 -> 22.5 ms on config 1).
+  // 119.0 -> 115.6 ms on volumes 1440p, 22.9 -> 22.5 on instancing 1080p).
   cswap(d0, l0, d1, l1);
   cswap(d2, l2, d3, l3);
   cswap(d0, l0, d2, l2);

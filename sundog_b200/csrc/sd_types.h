@@ -130,19 +130,18 @@ struct __align__(16) BvhNode {
 
 // Node layout the traversal reads: 1 (default) the 4-wide nodes below,
 // collapsed from the binary build; 0 the binary nodes themselves (measured
-// on the bench frames, Mrays/s, 4-wide / binary: config 1 1,652 / 1,622,
-// config 0 2,772 / 2,747, config 2 2,491 / 2,424).
+// on the bench frames, Mrays/s, 4-wide / binary: instancing 1,652 /
+// 1,622, Cornell 2,772 / 2,747, volumes 2,491 / 2,424).
 #ifndef SDB_BVH4
 #define SDB_BVH4 1
 #endif
 
 // 4-wide node (128 bytes, seven 16-byte loads), collapsed from the binary
 // tree on the device (bvh_device.cu: each node holds the grandchildren of
-// one binary node, or its child where that child is a leaf): the boxes of
-// children 0-1 and of children 2-3 each in BvhNode's box layout (so a pair
-// is tested with the binary node's arithmetic while the other pair is not
-// yet loaded), then the four links (inner node index >= 0, leaf code < 0 as
-// in BvhNode). An unused slot has the far point (3e30, 3e30, 3e30) as its
+// one binary node, or its child where that child is a leaf): the four
+// children's planes by axis and side, so a ray reads the near and far planes
+// of all of them by the signs of its direction, then the four links (inner
+// node index >= 0, leaf code < 0 as in BvhNode). An unused slot has the far point (3e30, 3e30, 3e30) as its
 // box, which no ray reaches within its tmax.
 struct __align__(128) Bvh4Node {
   float4 plane[6];  // lo.x hi.x lo.y hi.y lo.z hi.z of children 0-3

@@ -21,8 +21,9 @@
 // between stages (about 200 bytes per path segment).
 //
 // The stages call the megakernel's own per-path functions in the same order
-// with the same random draws, so every sample is the same sample as in
-// ptPersistent, and the film fold is unchanged.
+// with the same random draws, so every sample is ptPersistent's up to FP32
+// rounding (Rounding, sd_bsdf.cuh: a path may part from the megakernel's in
+// its last bits; test_gpu_entry_points.py), and the film fold is the same.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -64,8 +65,10 @@ constexpr int kRound = (GUIDE & kWfServe) ? kRoundServe : kRoundStage;  // sd_bs
 #ifndef SDB_WF_TRACE_BLOCKS
 #define SDB_WF_TRACE_BLOCKS 8
 #endif
-// Resident blocks per SM the stage kernels are compiled for: traversal 8 ->
-// 64 registers, shading 5 -> 102 registers.
+// Resident blocks per SM the stage kernels are compiled for: traversal 8 of
+// 128 threads (64 registers), the flame march and late vertices 5 (up to 96),
+// shading 2 of 384 (80 registers, 228 bytes of spill stores and 304 of loads;
+// 320 threads at 102 registers: instancing 1080p 90.6 against 89.1 ms).
 #ifndef SDB_WF_LATE_BLOCKS
 #define SDB_WF_LATE_BLOCKS 5
 #endif
@@ -239,7 +242,7 @@ __device__ __forceinline__ int travKind(const BinTrav& t) {
 // frame with the one-action loop: 894 Mrays/s at 24, 869 with a grid-stride
 // loop, 752 when every idle lane fetches at once: fresh rays at the TLAS
 // root diverge from the warp's deep BLAS walks; with the 4-wide walk and
-// descent runs, config 1 / config 0: 1,717 / 2,798 at 20, 1,706 / 2,801 at
+// descent runs, instancing 1080p / Cornell 256x256: 1,717 / 2,798 at 20, 1,706 / 2,801 at
 // 24, 1,678 / 2,799 at 28).
 #ifndef SDB_WF_FETCH_IDLE
 #define SDB_WF_FETCH_IDLE 20
@@ -249,11 +252,12 @@ __device__ __forceinline__ int travKind(const BinTrav& t) {
 // Efficiency of Ray Traversal on GPUs", 2009): the traversal loop runs per
 // warp, and a lane whose ray is done writes its hit and, once
 // SDB_WF_FETCH_IDLE lanes of the warp are idle, takes the next ray of the
-// live list (one warp-aggregated atomicAdd on counts[3]), so a warp no longer
+// live list (one warp-aggregated atomicAdd on fetchRay), so a warp no longer
 // waits for its longest ray. Each ray visits the nodes of traverse<false>
 // (sd_trace.cuh) in the same order with the same tests: the same closest
-// accepted hit. (Shadow rays, shorter, gained nothing from it.) SERVE: a
-// serving batch, each lane tracing in its own job's scene.
+// accepted hit. (Shadow rays take the same form in scenes of many instances,
+// wfShadowFetch.) SERVE: a serving batch, each lane tracing in its own job's
+// scene.
 #if SDB_WIDE_BVH
 // The same stage over the compressed 8-wide BVH (CwNode, sd_trace.cuh): each
 // loop iteration a lane either tests one primitive of its current leaf group
@@ -819,7 +823,7 @@ template <int GUIDE, bool CAM>
 __global__ void __launch_bounds__(kShadeBlock, SDB_WF_SHADE_BLOCKS) wfShade(
     int it, int depth, unsigned long long base) {
   __shared__ int sSlot[kTileMax];
-  __shared__ unsigned short sKey[kTileMax];    // class << 8 | rank; then the sorted order
+  __shared__ unsigned short sKey[kTileMax];    // class << 8 | rank
   __shared__ unsigned char sFlag[kTileMax];
   __shared__ unsigned short sOrder[kTileMax];
   constexpr int kGroups = kTileMax / 32;       // warps' worth of entries in a tile
@@ -1008,8 +1012,8 @@ struct ShadowSink {
 // Shadow rays with the trace stage's dynamic fetch and
 // node-descent runs: the walk and transmittance of shadowTransmittance, many
 // rays interleaved per warp. Faster than wfShadow where walks are long and
-// uneven (config 1, 1024 instances: 29.3 -> 24.5 ms per frame), slower on
-// small scenes (config 0: 2,730 -> 2,672 Mrays/s; config 2: 113.7 -> 122.2
+// uneven (1024 instances, 1080p: 29.3 -> 24.5 ms per frame), slower on small
+// scenes (Cornell: 2,730 -> 2,672 Mrays/s; volumes 1440p: 113.7 -> 122.2
 // ms), so renders choose by instance count (kShadowFetchInstances).
 template <int GUIDE>
 __global__ void __launch_bounds__(kRenderBlock, SDB_WF_TRACE_BLOCKS) wfShadowFetch(int it, int depth) {
