@@ -872,9 +872,8 @@ void RenderSession::render(cudaStream_t st, bool reset, sundog_render_result* re
         // A tile shard that owns no tile: nothing to trace.
       } else if (wavefront) {
         if (!wf) wf = wfAcquire();
-        const int slots = (int)std::min<unsigned long long>(lp.numPaths, kWavefrontSlots);
-        wf->ensure(slots);
-        if (wfHasLate(lp, mode)) wf->ensureLate(slots);
+        wf->ensure((int)std::min<unsigned long long>(lp.numPaths, kWavefrontSlots),
+                   wfHasLate(lp, mode));
         launches += wfRender(lp, *wf, st, mode, stageTiming ? &stages : nullptr);
       } else {
         cudaCheck(launchRender(st, grid, mode), "path kernel launch");

@@ -163,7 +163,7 @@ class Server {
       wf = wfAcquire();
       uint64_t batchPaths = cfg.iteration_paths + (uint64_t)kMaxServeJobs * maxItemPaths;
       batchSlots = (int)std::min<uint64_t>(batchPaths, 1ull << 26);
-      wf->ensure(batchSlots);
+      wf->ensure(batchSlots, false);
     }
     slots.assign(kMaxServeJobs, nullptr);
     thread = std::thread([this] { loop(); });

@@ -1175,26 +1175,33 @@ bool wfHasLate(const SdLaunch& lp, int guide) {
   return (guide & kGuideRecord) || (lp.numFlames > 0 && lp.transparentShadows);
 }
 
-void WfBuffers::ensure(int slots) {
-  if (slots <= cap) return;
+void WfBuffers::ensure(int slots, bool withLate) {
+  if (slots > cap) grow(slots, withLate);
+  if (withLate) ensureLate(slots);
+}
+
+void WfBuffers::grow(int slots, bool withLate) {
   // At most half of the device memory that is free (counting the pool about
   // to be replaced), so films, scenes and other work keep room; at least
   // 1 M slots.
   size_t freeB = 0, totB = 0;
   cudaCheck(cudaMemGetInfo(&freeB, &totB), "cudaMemGetInfo");
-  const size_t budget = (freeB + (size_t)cap * wfSlotBytes()) / 2;
-  const size_t fit = std::max<size_t>(budget / wfSlotBytes(), (size_t)1 << 20);
+  const bool within = withLate && !verts.ptr;  // late vertices in the slab
+  const size_t per = wfSlotBytes() + (within ? wfLateBytes() : 0);
+  const size_t fit = std::max<size_t>((freeB + slab.bytes) / 2 / per, (size_t)1 << 20);
   slots = (int)std::min<size_t>((size_t)slots, fit);
   if (slots <= cap) return;
   const size_t n = (size_t)slots;
-  const size_t sizes[11] = {n * 32, n * 32, n * 32, n * 32, n * 32, n * 16,
-                            n * sizeof(int), n * sizeof(int), n * sizeof(int), n * sizeof(int), n};
-  size_t offs[11], total = 0;
-  for (int k = 0; k < 11; k++) {
+  const size_t sizes[12] = {n * 32, n * 32, n * 32, n * 32, n * 32, n * 16,
+                            n * sizeof(int), n * sizeof(int), n * sizeof(int), n * sizeof(int), n,
+                            within ? n * wfLateBytes() : 0};
+  size_t offs[12], total = 0;
+  for (int k = 0; k < 12; k++) {
     offs[k] = total;
     total += (sizes[k] + 255) & ~(size_t)255;
   }
   cap = 0;
+  if (!verts.ptr) lateCap = 0;  // those in the slab go with it
   slab.release();
   slab.alloc(total);
   char* base = (char*)slab.ptr;
@@ -1209,6 +1216,10 @@ void WfBuffers::ensure(int slots) {
   pool.shadowList = (int*)(base + offs[8]);
   pool.lateList = (int*)(base + offs[9]);
   pool.jobs = (unsigned char*)(base + offs[10]);
+  if (within) {
+    pool.verts = (PoolSlot<LateVertex>*)(base + offs[11]);
+    lateCap = slots;
+  }
   if (!counts.ptr) counts.alloc((kWfGroup + 1) * sizeof(WfCounts));
   pool.counts = (WfCounts*)counts.ptr;
   if (!hostCount) hostCount = pinnedWords();
@@ -1229,18 +1240,19 @@ void WfBuffers::ensure(int slots) {
 void WfBuffers::ensureLate(int slots, size_t keep) {
   slots = std::min(slots, cap);
   if (slots <= lateCap) return;
-  // A buffer of its own, for the paths of the launches that have late
-  // vertices: a pool kept from a large frame is not made again for them.
-  // Half of the free memory at most, as the pool's.
+  // A buffer of its own: a pool kept from a large frame is not made again for
+  // the late vertices of a small one. Half of the free memory at most, as the
+  // pool's.
   size_t freeB = 0, totB = 0;
   cudaCheck(cudaMemGetInfo(&freeB, &totB), "cudaMemGetInfo");
-  freeB += (size_t)lateCap * wfLateBytes();
+  freeB += verts.bytes;
   const size_t fit = std::max<size_t>((freeB > keep ? freeB - keep : 0) / 2 / wfLateBytes(),
                                       (size_t)1 << 20);
   slots = (int)std::min<size_t>((size_t)slots, fit);
   if (slots <= lateCap) return;
   lateCap = 0;
   verts.alloc((size_t)slots * wfLateBytes());
+  pool.verts = (PoolSlot<LateVertex>*)verts.ptr;
   lateCap = slots;
 }
 
@@ -1382,7 +1394,6 @@ static int runPool(WfBuffers& b, cudaStream_t st, unsigned long long numPaths, c
     for (cudaEvent_t& e : b.ev) cudaCheck(cudaEventCreate(&e), "stage timing events");
   WfPool pool = b.pool;
   pool.trails = (PoolSlot<GuideTrail>*)b.trails.ptr;
-  pool.verts = (PoolSlot<LateVertex>*)b.verts.ptr;
   // Paths in flight at once: slots, with a late vertex each where there can be some.
   const int cap = plan.late ? std::min(b.cap, b.lateCap) : b.cap;
   if (cap < 1) throw std::runtime_error("wavefront: no path slots");

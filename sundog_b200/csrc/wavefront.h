@@ -50,7 +50,7 @@ struct WfPool {
   float4* hits;               // two: t, inst, prim | media << 30 | front << 31, u / v, normal.xyz
   float4* shadowRays;         // two: origin.xyz dir.xyz, tmax, flags
   float4* shadowTerms;        // the NEE term; for a late vertex its transmittance
-  PoolSlot<LateVertex>* verts;  // late vertices, in a buffer of their own (WfBuffers::ensureLate)
+  PoolSlot<LateVertex>* verts;  // late vertices (WfBuffers::lateCap slots have one)
   int* lists[2];              // live slot lists, ping-pong between iterations
   int *shadowList;
   int *lateList;              // late vertices; before shading, the rays that may meet a flame
@@ -66,13 +66,13 @@ struct WfBuffers {
   DevBuf slab, counts;
   WfPool pool = {};
   DevBuf trails;  // allocated by the first training-record pass
-  DevBuf verts;   // late vertices, from the first launch that may have some
+  DevBuf verts;   // late vertices, where the slab was made without them
   unsigned* hostCount = nullptr;   // pinned: counters read back (from a process-wide free list)
   cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};  // stage timing
   cudaStream_t side = nullptr;  // the shadow stage's, beside the next trace
   cudaEvent_t shaded = nullptr, shadowDone = nullptr;
   int cap = 0;
-  int lateCap = 0;   // slots with room for a late vertex
+  int lateCap = 0;   // slots with room for a late vertex, in the slab or in verts
   int trailCap = 0;
   int gridStart = 0, gridTrace = 0, gridShade = 0, gridShadow = 0, gridLate = 0,
       gridFlame = 0;
@@ -80,12 +80,16 @@ struct WfBuffers {
   WfBuffers(const WfBuffers&) = delete;
   WfBuffers& operator=(const WfBuffers&) = delete;
   ~WfBuffers();
-  // Room for `slots` paths (fewer when device memory is short).
-  void ensure(int slots);
-  // Room for the late vertices of `slots` of them (fewer when device memory
-  // is short; `keep` bytes of it are left free).
+  // Room for `slots` paths (fewer when device memory is short), and with
+  // withLate for their late vertices: in the slab where it is made now.
+  void ensure(int slots, bool withLate);
+  // Room for the late vertices of `slots` of the pool's paths (fewer when
+  // device memory is short; `keep` bytes of it are left free).
   void ensureLate(int slots, size_t keep = 0);
   void ensureTrails();  // one GuideTrail per slot
+
+ private:
+  void grow(int slots, bool withLate);
 };
 
 // Whether paths of the launch may have late vertices: those whose next draws
