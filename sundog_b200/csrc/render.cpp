@@ -857,8 +857,14 @@ void RenderSession::render(cudaStream_t st, bool reset, sundog_render_result* re
     }
     lp.sampleOffset = sampleBase + done;
     lp.sppThisLaunch = n;
-    lp.sampleMajor = (mode & kGuideRecord) ? 1 : 0;
     lp.numPaths = (unsigned long long)pathsPerSample(lp) * n;
+    // A film that is mostly tile padding (a row, a column, a pixel): the
+    // megakernel's warps would hold all samples of a pixel or none. Samples
+    // outermost give each a share (101x1 at 16 samples: instancing 276 -> 210
+    // us, features 199 -> 134; a whole pixel per warp is better from 17x9 on,
+    // features at 64 samples 363 against 474).
+    const bool sparse = engine == 1 && (unsigned long long)pathsPerSample(lp) >= 4 * shardPixels;
+    lp.sampleMajor = (mode & kGuideRecord) || sparse ? 1 : 0;
     cudaCheck(cudaMemsetAsync(lp.pathCounter, 0, sizeof(unsigned long long), st), "counter reset");
     {
       // The launch blocks live in per-device constant memory: hold the

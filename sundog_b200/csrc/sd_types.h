@@ -204,7 +204,7 @@ struct SdLaunch {
   // work decomposition: path p -> (tile-ordered pixel p / sppThisLaunch, sample);
   // sampleMajor: (sample, pixel) instead, for launches that keep the training
   // records of the paths that end first (the record cap then cuts samples,
-  // not a part of the image)
+  // not a part of the image) and megakernel launches of mostly padding
   int sampleMajor;
   int tilesX;
   int npixPad;
