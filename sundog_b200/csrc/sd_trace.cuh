@@ -622,17 +622,19 @@ __device__ __forceinline__ int binTravInstance(BinTrav& t, TravStack& stack, con
   if (in.kind == GK_MESH) {
     if (COUNT) cnt->blasEntries++;
     // Always room: the scene build bounds TLAS + BLAS depth by the stack.
-    if (t.sp >= kStackSize) return binTravEnd<POP>(t, stack, sink);
-    stack[t.sp++] = kToTlas;
-    t.inBlas = true;
-    t.curInst = start;
-    t.ro = o2;
-    t.rd = d2;
-    t.id = v3(safeInv(d2.x), safeInv(d2.y), safeInv(d2.z));
-    t.oi = o2 * t.id;
-    t.wr = wtSetup(d2);
-    t.cur = lp.meshes[in.mesh].root;
-    return kTravMore;
+    if (t.sp < kStackSize) {
+      stack[t.sp++] = kToTlas;
+      t.inBlas = true;
+      t.curInst = start;
+      t.ro = o2;
+      t.rd = d2;
+      t.id = v3(safeInv(d2.x), safeInv(d2.y), safeInv(d2.z));
+      t.oi = o2 * t.id;
+      t.wr = wtSetup(d2);
+      t.cur = lp.meshes[in.mesh].root;
+      return kTravMore;
+    }
+    return binTravEnd<POP>(t, stack, sink);
   }
   if (COUNT) cnt->quadTests++;
   QHits qh = hitQuadric(in.kind, o2, d2, tmin, t.tmax);

@@ -57,6 +57,7 @@ struct WfPool {
   WfCounts* counts;           // kWfGroup + 1
   PoolSlot<GuideTrail>* trails;  // guided vertices awaiting their path's end (record passes)
   unsigned char* jobs;        // serving batches: the job slot of each slot's path
+  unsigned long long* seen;   // host memory: the last report (wfReport)
 };
 
 // Host-owned pool storage, grown on demand.
@@ -67,7 +68,8 @@ struct WfBuffers {
   WfPool pool = {};
   DevBuf trails;  // allocated by the first training-record pass
   DevBuf verts;   // late vertices, where the slab was made without them
-  unsigned* hostCount = nullptr;   // pinned: counters read back (from a process-wide free list)
+  // Pinned words, from a process-wide free list: counters read back, WfPool::seen.
+  unsigned *hostCount = nullptr, *hostSeen = nullptr;
   cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};  // stage timing
   cudaStream_t side = nullptr;  // the shadow stage's, beside the next trace
   cudaEvent_t shaded = nullptr, shadowDone = nullptr;
